@@ -11,8 +11,8 @@
 // Work is bucketed by net size; every bucket is one persistent launch whose
 // CTAs pull nets from a device-side queue (no host round trip, graph
 // capturable):
-//   * nets of <= 32 nodes: one warp per net, one lane per node, all in
-//     registers and shuffles;
+//   * nets of <= 32 nodes: eight nets per warp, four lanes each
+//     (otg_rc_small.cuh);
 //   * larger nets: one CTA per net, staged in shared memory (or, for nets
 //     beyond the shared-memory budget, in a per-CTA slice of the caller's
 //     workspace, which stays L2-resident).  The tree is processed with
@@ -112,190 +112,23 @@ __device__ __forceinline__ float sink_slew1(float si, float imp) {
   return si < 0.0f ? -r : r;
 }
 
-__device__ __forceinline__ float4 f4add(float4 a, float4 b) {
-  return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+// Size checks of one job item: the net's node count, or -1 after reporting
+// a net that is out of range, empty or larger than the caller declared.
+__device__ __forceinline__ int job_net_size(const RcArgs& a, int net) {
+  return a.nodes_start[net + 1] - a.nodes_start[net];
 }
-__device__ __forceinline__ float4 f4mul(float4 a, float4 b) {
-  return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w);
+__device__ __forceinline__ int checked_net_size(const RcArgs& a, int net, int item,
+                                                int max_net_nodes, int* status) {
+  const int n = (unsigned)net < (unsigned)a.num_nets ? job_net_size(a, net) : 0;
+  if (n >= 1 && n <= max_net_nodes) return n;
+  if (atomicCAS(status, 0, n < 1 ? OTG_ERR_INVALID : OTG_ERR_TOO_LARGE) == 0) status[1] = item;
+  return -1;
 }
-__device__ __forceinline__ float4 f4scale(float4 a, float s) {
-  return make_float4(a.x * s, a.y * s, a.z * s, a.w * s);
-}
-__device__ __forceinline__ float4 shfl4(float4 v, int src) {
-  return make_float4(__shfl_sync(FULL, v.x, src), __shfl_sync(FULL, v.y, src),
-                     __shfl_sync(FULL, v.z, src), __shfl_sync(FULL, v.w, src));
-}
-
-// =====================================================================
-// Warp path: nets of <= 32 nodes.  Lane v holds node v and edge v.
-// =====================================================================
-__device__ void rc_net_warp(const RcArgs& a, int net, int* s_par, int* s_pe) {
-  const int lane = threadIdx.x & 31;
-  const int b = a.nodes_start[net];
-  const int n = a.nodes_start[net + 1] - b;
-  const int m = n - 1;
-  const int eb = b - net;
-  const int root = a.roots[net];
-  const bool isnode = lane < n;
-  const bool isedge = lane < m;
-
-  int es = 0, et = 0;
-  float r = 0.0f;
-  if (isedge) {
-    int2 e = a.edges[eb + lane];
-    es = e.x;
-    et = e.y;
-    r = a.res[eb + lane];
-  }
-  float4 cap = isnode ? a.cap[b + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const bool bad = (isedge && ((unsigned)es >= (unsigned)n || (unsigned)et >= (unsigned)n)) ||
-                   (unsigned)root >= (unsigned)n;
-  if (__any_sync(FULL, bad)) {
-    if (lane == 0) report(a, OTG_ERR_INVALID, net);
-    return;
-  }
-
-  // Level-synchronous BFS from the root (depth <= 31).
-  constexpr int INF = 1 << 20;
-  int dist = (lane == root) ? 0 : INF;
-  int my_par = -1, my_child = -1;
-  s_par[lane] = -1;
-  s_pe[lane] = -1;
-  __syncwarp();
-  for (int level = 0; level < n; ++level) {
-    int ds = __shfl_sync(FULL, dist, es);
-    int dt = __shfl_sync(FULL, dist, et);
-    int child = -1, par = -1;
-    if (isedge) {
-      if (ds == level && dt == INF) { child = et; par = es; }
-      else if (dt == level && ds == INF) { child = es; par = et; }
-    }
-    unsigned D = __reduce_or_sync(FULL, child >= 0 ? (1u << child) : 0u);
-    if (child >= 0) {
-      s_par[child] = par;
-      s_pe[child] = lane;
-      my_par = par;
-      my_child = child;
-    }
-    if ((D >> lane) & 1u) dist = level + 1;
-    if (D == 0u) break;
-  }
-  __syncwarp();
-  const unsigned reached = __ballot_sync(FULL, isnode && dist < INF);
-  const unsigned want = (n == 32) ? FULL : ((1u << n) - 1u);
-  if (reached != want) {
-    if (lane == 0) report(a, OTG_ERR_NOT_TREE, net);
-    return;
-  }
-  int parent = s_par[lane];
-  if (lane == root || !isnode) parent = lane;
-
-  // BFS slot: (dist asc, local id desc) -- ot/cuda/sort.cuh:102-121.
-  int slot = 0;
-  for (int u = 0; u < n; ++u) {
-    int du = __shfl_sync(FULL, dist, u);
-    slot += (du < dist) || (du == dist && u > lane);
-  }
-  const int pslot = __shfl_sync(FULL, slot, parent);
-  if (isnode) {
-    a.node2bfs[b + lane] = slot;
-    a.pid[b + slot] = slot - pslot;  // root: 0
-  }
-  if (isedge) a.edges[eb + lane] = make_int2(my_par, my_child);
-
-  // Ancestor-or-self masks by pointer doubling.
-  unsigned M = isnode ? ((1u << lane) | (1u << parent)) : 0u;
-  int anc = parent;
-  for (int k = 0; k < 5; ++k) {
-    unsigned Ma = __shfl_sync(FULL, M, anc);
-    int aa = __shfl_sync(FULL, anc, anc);
-    M |= Ma;
-    anc = aa;
-  }
-  // pres of node v = resistance of the edge to its parent
-  float pres = 0.0f;
-  {
-    int pe = (isnode && lane != root) ? s_pe[lane] : 0;
-    float rr = __shfl_sync(FULL, r, pe);
-    pres = (isnode && lane != root) ? rr : 0.0f;
-  }
-  // load: sum of cap over the subtree (descendants u have bit v in M[u])
-  float4 load = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int u = 0; u < n; ++u) {
-    unsigned Mu = __shfl_sync(FULL, M, u);
-    float4 c = shfl4(cap, u);
-    if ((Mu >> lane) & 1u) load = f4add(load, c);
-  }
-  // delay: sum of pres*load over ancestors-or-self
-  float4 w = f4scale(load, pres);
-  float4 delay = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int u = 0; u < n; ++u) {
-    float4 wu = shfl4(w, u);
-    if ((M >> u) & 1u) delay = f4add(delay, wu);
-  }
-  float4 x = f4mul(cap, delay);
-  float4 ldelay = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int u = 0; u < n; ++u) {
-    unsigned Mu = __shfl_sync(FULL, M, u);
-    float4 c = shfl4(x, u);
-    if ((Mu >> lane) & 1u) ldelay = f4add(ldelay, c);
-  }
-  w = f4scale(ldelay, pres);
-  float4 beta = make_float4(0.f, 0.f, 0.f, 0.f);
-  for (int u = 0; u < n; ++u) {
-    float4 wu = shfl4(w, u);
-    if ((M >> u) & 1u) beta = f4add(beta, wu);
-  }
-  float4 imp = make_float4(fmaf(-delay.x, delay.x, 2.0f * beta.x),
-                           fmaf(-delay.y, delay.y, 2.0f * beta.y),
-                           fmaf(-delay.z, delay.z, 2.0f * beta.z),
-                           fmaf(-delay.w, delay.w, 2.0f * beta.w));
-  if (isnode) {
-    a.load[b + slot] = load;
-    a.delay[b + slot] = delay;
-    a.ldelay[b + slot] = ldelay;
-    a.impulse[b + slot] = imp;
-  }
-  if (a.sinks_start) {
-    const int s0 = a.sinks_start[net], s1 = a.sinks_start[net + 1];
-    const float4 si = a.driver_slew[net];
-    for (int k0 = s0; k0 < s1; k0 += 32) {
-      int k = k0 + lane;
-      int v = k < s1 ? a.sink_nodes[k] : 0;
-      bool ok = k < s1 && (unsigned)v < (unsigned)n;
-      float4 iv = shfl4(imp, ok ? v : 0);
-      if (ok) {
-        float4 o;
-        o.x = sink_slew1(si.x, iv.x);
-        o.y = sink_slew1(si.y, iv.y);
-        o.z = sink_slew1(si.z, iv.z);
-        o.w = sink_slew1(si.w, iv.w);
-        a.sink_slew[k] = o;
-      } else if (k < s1) {
-        report(a, OTG_ERR_INVALID, net);
-      }
-    }
-  }
+__device__ __forceinline__ void check_job_count(const RcJob& job, int cap, int* status) {
+  if (job_count(job) > cap && atomicCAS(status, 0, OTG_ERR_WORKSPACE) == 0) status[1] = -1;
 }
 
-__global__ void __launch_bounds__(256) rc_warp_kernel(RcJob job, const int* list,
-                                                       const int* count, int* work) {
-  __shared__ int s_par[8][32];
-  __shared__ int s_pe[8][32];
-  const int w = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int cnt = *count;
-  while (true) {
-    int item = 0;
-    if (lane == 0) item = atomicAdd(work, 1);
-    item = __shfl_sync(FULL, item, 0);
-    if (item >= cnt) break;
-    int f, net;
-    job_item(job, list[item], f, net);
-    rc_net_warp(job_forest(job, f), net, s_par[w], s_pe[w]);
-    __syncwarp();
-  }
-}
+#include "otg_rc_small.cuh"
 
 // Optional per-phase cycle accounting (build with -DOTG_PHASE_TIMING; the
 // product build compiles it out).  Thread 0 of each CTA adds the clock64()
@@ -1225,18 +1058,13 @@ __global__ void rc_classify_kernel(RcJob job, int cap, int max_net_nodes, RcClas
   if (i < num) {
     int f, net;
     job_item(job, i, f, net);
-    const RcArgs& a = job_forest(job, f);
-    const int n = (unsigned)net < (unsigned)a.num_nets
-                      ? a.nodes_start[net + 1] - a.nodes_start[net] : 0;
-    if (n < 1 || n > max_net_nodes) {
-      if (atomicCAS(status, 0, n < 1 ? OTG_ERR_INVALID : OTG_ERR_TOO_LARGE) == 0) status[1] = i;
-    } else {
+    const int n = checked_net_size(job_forest(job, f), net, i, max_net_nodes, status);
+    if (n > 0) {
       c = 0;
       while (c < cls.num - 1 && n > cls.nmax[c]) ++c;
     }
   }
-  if (i == 0 && job_count(job) > cap && atomicCAS(status, 0, OTG_ERR_WORKSPACE) == 0)
-    status[1] = -1;
+  if (i == 0) check_job_count(job, cap, status);
   // warp-aggregated append of the item index
   const unsigned active = __ballot_sync(FULL, c >= 0);
   const unsigned peers = __match_any_sync(FULL, c);
@@ -1274,8 +1102,8 @@ DevInfo& dev_info() {
 // kernel (sh[], s_item: under 1 KB).
 constexpr int kStaticSmemReserve = 2048;
 
-// Size classes.  Class 0: the warp path (nets of <= 32 nodes; its
-// lane-per-node scheme fixes that bound).  Classes 1..6: one CTA per net in
+// Size classes.  Class 0: the small-net kernel (its adjacency masks fix its
+// bound of 32 nodes).  Classes 1..6: one CTA per net in
 // shared memory (16-bit indices); their upper bounds and tile shapes (T
 // threads, K scan items per thread) come from the device's tuning.
 // Class 7: nets beyond the last block class, in per-CTA slices of the
@@ -1360,7 +1188,7 @@ bool tune_ok(const RcTune& t, int smem_budget) {
 RcClasses classes_of(const RcTune& t) {
   RcClasses c;
   c.num = RcClasses::kMax;
-  c.nmax[0] = 32;
+  c.nmax[0] = kSmallMax;
   for (int k = 1; k <= kBlockClasses; ++k) c.nmax[k] = t.nmax[std::min(k, t.num) - 1];
   c.nmax[RcClasses::kMax - 1] = 1 << 30;
   return c;
@@ -1567,6 +1395,11 @@ bool forest_ok(const otg_rc_forest* f) {
 
 }  // namespace
 
+// CTAs of the small-net kernel: one warp and eight nets each at a time.
+int small_ctas(int nets, int sms) {
+  return std::max(1, std::min((nets + 7) / 8, kSmallCtas * sms));
+}
+
 // Launches the fused pass over the items of `job` (at most `cap` of them).
 // The workspace starts with [status 64 B][counters 64 B]; its status word is
 // where a.status should point for single-forest jobs.
@@ -1592,6 +1425,15 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
     return OTG_ERR_CUDA;
   }
   if (cap == 0) return OTG_OK;
+  // every net is small: no classes to sort into (sorting 250,000 nets takes
+  // 9 us, and a call of 64 nets a third of its launches)
+  if (max_net_nodes <= kSmallMax) {
+    rc_small_kernel<<<small_ctas(cap, di.sms), 32, 0, stream>>>(
+        job, nullptr, nullptr, cap, max_net_nodes, status);
+    count_launch();
+    if (cudaGetLastError() != cudaSuccess) return OTG_ERR_CUDA;
+    return OTG_OK;
+  }
   rc_classify_kernel<<<(cap + 255) / 256, 256, 0, stream>>>(job, cap, max_net_nodes, cls, lists,
                                                             counters, status);
   count_launch();
@@ -1646,7 +1488,8 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
                        next_stream());
   }
   if (err == cudaSuccess) {
-    rc_warp_kernel<<<di.sms * 8, 256, 0, next_stream()>>>(job, L(0), counters + 0, work + 0);
+    rc_small_kernel<<<small_ctas(cap, di.sms), 32, 0, next_stream()>>>(
+        job, L(0), counters + 0, cap, max_net_nodes, status);
     count_launch();
     err = cudaGetLastError();
   }
