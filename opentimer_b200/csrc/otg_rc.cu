@@ -128,6 +128,21 @@ __device__ __forceinline__ void check_job_count(const RcJob& job, int cap, int* 
   if (job_count(job) > cap && atomicCAS(status, 0, OTG_ERR_WORKSPACE) == 0) status[1] = -1;
 }
 
+// The class kernels of one pass are launched so that each may start as soon
+// as every CTA of the one before it has (programmatic dependent launch):
+// the classes are independent, and one class's last nets leave most SMs
+// idle.  chain_next() lets the next kernel start; chain_end() keeps this one
+// from completing before the one ahead of it has, so the last kernel's
+// completion is the whole pass's.  Only the first CTA waits there, so no
+// other holds its SM's shared memory.  A kernel launched the ordinary way
+// passes through both.
+__device__ __forceinline__ void chain_next() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chain_end() {
+  if (blockIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 #include "otg_rc_small.cuh"
 
 // Optional per-phase cycle accounting (build with -DOTG_PHASE_TIMING; the
@@ -979,8 +994,8 @@ __global__ void __launch_bounds__(T) rc_block_kernel(RcJob job, const int* list,
   __shared__ RcArgs s_args;  // the current net's forest
   char* ws = SMEM ? dsm : gws + (size_t)blockIdx.x * ws_stride;
   const int cnt = *count;
-  if (cnt <= few) return;
-  while (true) {
+  chain_next();
+  while (cnt > few) {
     if (threadIdx.x == 0) {
       const int item = atomicAdd(work, 1);
       s_item[0] = item;
@@ -1001,6 +1016,7 @@ __global__ void __launch_bounds__(T) rc_block_kernel(RcJob job, const int* list,
                                 CtaGroup<T>{sh + 32, sh + 33, (unsigned*)(sh + 40)});
     __syncthreads();
   }
+  chain_end();
 }
 
 // Nets above the shared-memory classes, one thread-block cluster per net:
@@ -1032,8 +1048,9 @@ __global__ void __launch_bounds__(T) rc_cluster_kernel(RcJob job, const int* lis
   g.smx = (unsigned*)cl.map_shared_rank(sh + 40, 0);
   g.xch = xch;
   const int cnt = *count;
-  if (cnt > few) return;  // uniform: no CTA has touched another's memory
-  for (int item = cid; item < cnt; item += ncl) {
+  chain_next();
+  // more than `few`: none (uniform, no CTA has touched another's memory)
+  for (int item = cid; item < cnt && cnt <= few; item += ncl) {
     if (threadIdx.x == 0) {
       int f, net;
       job_item(job, list[item], f, net);
@@ -1046,6 +1063,7 @@ __global__ void __launch_bounds__(T) rc_cluster_kernel(RcJob job, const int* lis
     rc_net_block<T, K, int>(s_args, net, ws, n, sh, shl, g);
     g.sync();  // the slice, s_args and rank 0's scalars are reused by the next item
   }
+  chain_end();
 }
 
 // ------------------------------------------------------------ bucketing
@@ -1322,9 +1340,35 @@ size_t rc_workspace_bytes(int num_nets, int max_net_nodes, int sms, int smem_bud
 
 namespace {
 
+// Launches one kernel of a pass's chain; `chained`: it may start before the
+// launch ahead of it on the stream has completed (see chain_next).
+template <class... P, class... A>
+cudaError_t chain_launch(void (*kern)(P...), int grid, int block, size_t smem, int cluster,
+                         bool chained, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  if (cluster > 1) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    at[cfg.numAttrs].val.clusterDim.x = (unsigned)cluster;
+    at[cfg.numAttrs].val.clusterDim.y = 1;
+    at[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
+  if (chained) {
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  count_launch();
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 template <int T, int K>
 cudaError_t launch_smem_class(const RcJob& job, const int* list, int* count, int* work, int nmax,
-                              int sms, cudaStream_t stream) {
+                              int sms, bool chained, cudaStream_t stream) {
   const bool tile = rc_use_tile();
   auto kern = tile ? rc_block_kernel<T, K, uint16_t, true, true> : rc_block_kernel<T, K, uint16_t, true>;
   const size_t smem = rc_smem_bytes(nmax, T, K, tile);
@@ -1336,26 +1380,25 @@ cudaError_t launch_smem_class(const RcJob& job, const int* list, int* count, int
   if (err == cudaSuccess) err = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T, smem);
   if (err != cudaSuccess) return err;
   occ = std::max(occ, 1);
-  kern<<<sms * occ, T, smem, stream>>>(job, list, count, work, nullptr, 0, 0);
-  count_launch();
-  return cudaGetLastError();
+  return chain_launch(kern, sms * occ, T, smem, 1, chained, stream, job, list, count, work,
+                      nullptr, 0, 0);
 }
 
 cudaError_t launch_shape(int s, const RcJob& job, const int* list, int* count, int* work,
-                         int nmax, int sms, cudaStream_t st) {
+                         int nmax, int sms, bool chained, cudaStream_t st) {
   switch (s) {
-    case 0: return launch_smem_class<64, 4>(job, list, count, work, nmax, sms, st);
-    case 1: return launch_smem_class<64, 8>(job, list, count, work, nmax, sms, st);
-    case 2: return launch_smem_class<128, 4>(job, list, count, work, nmax, sms, st);
-    case 3: return launch_smem_class<128, 8>(job, list, count, work, nmax, sms, st);
-    case 4: return launch_smem_class<256, 2>(job, list, count, work, nmax, sms, st);
-    case 5: return launch_smem_class<256, 4>(job, list, count, work, nmax, sms, st);
-    case 6: return launch_smem_class<256, 8>(job, list, count, work, nmax, sms, st);
-    case 7: return launch_smem_class<512, 2>(job, list, count, work, nmax, sms, st);
-    case 8: return launch_smem_class<512, 4>(job, list, count, work, nmax, sms, st);
-    case 9: return launch_smem_class<512, 8>(job, list, count, work, nmax, sms, st);
-    case 10: return launch_smem_class<1024, 2>(job, list, count, work, nmax, sms, st);
-    case 11: return launch_smem_class<1024, 4>(job, list, count, work, nmax, sms, st);
+    case 0: return launch_smem_class<64, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 1: return launch_smem_class<64, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 2: return launch_smem_class<128, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 3: return launch_smem_class<128, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 4: return launch_smem_class<256, 2>(job, list, count, work, nmax, sms, chained, st);
+    case 5: return launch_smem_class<256, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 6: return launch_smem_class<256, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 7: return launch_smem_class<512, 2>(job, list, count, work, nmax, sms, chained, st);
+    case 8: return launch_smem_class<512, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 9: return launch_smem_class<512, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 10: return launch_smem_class<1024, 2>(job, list, count, work, nmax, sms, chained, st);
+    case 11: return launch_smem_class<1024, 4>(job, list, count, work, nmax, sms, chained, st);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1444,8 +1487,11 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
   // stream and the side streams (joined back below), so the classes run
   // side by side instead of one after another.
   const int nside = fork ? std::min(fork->n, RcFork::kMax) : 0;
+  // Without one, every launch after the first joins the pass's chain.
   int nth = 0;
+  bool chained = false;
   auto next_stream = [&]() -> cudaStream_t {
+    chained = nside == 0 && nth > 0;
     const int k = nth++ % (nside + 1);
     return k == 0 ? stream : fork->side[k - 1];
   };
@@ -1459,39 +1505,24 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
     const HugePlan h = huge_plan(max_net_nodes, di.sms);
     const int few = h.S > 1 ? kClusterNetsPerCluster * h.clusters : 0;
     cudaStream_t hs = next_stream();
-    rc_block_kernel<kHugeT, kHugeK, int, false><<<h.ctas, kHugeT, 0, hs>>>(
-        job, L(7), counters + 7, work + 7, ws + off_huge, stride, few);
-    count_launch();
-    err = cudaGetLastError();
-    if (err == cudaSuccess && h.S > 1) {
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute at[1];
-      at[0].id = cudaLaunchAttributeClusterDimension;
-      at[0].val.clusterDim.x = (unsigned)h.S;
-      at[0].val.clusterDim.y = 1;
-      at[0].val.clusterDim.z = 1;
-      cfg.gridDim = dim3(h.clusters * h.S);
-      cfg.blockDim = dim3(kHugeT);
-      cfg.stream = hs;
-      cfg.attrs = at;
-      cfg.numAttrs = 1;
-      err = cudaLaunchKernelEx(&cfg, rc_cluster_kernel<kHugeT, kHugeK>, job, (const int*)L(7),
-                               (const int*)(counters + 7), ws + off_huge + stride * (size_t)h.ctas,
-                               h.stride_c, few);
-      count_launch();
-    }
+    err = chain_launch(rc_block_kernel<kHugeT, kHugeK, int, false>, h.ctas, kHugeT, 0, 1, chained,
+                       hs, job, L(7), counters + 7, work + 7, ws + off_huge, stride, few);
+    if (err == cudaSuccess && h.S > 1)
+      err = chain_launch(rc_cluster_kernel<kHugeT, kHugeK>, h.clusters * h.S, kHugeT, 0, h.S,
+                         nside == 0, hs, job, L(7), counters + 7,
+                         ws + off_huge + stride * (size_t)h.ctas, h.stride_c, few);
   }
   for (int c = tn.num; c >= 1 && err == cudaSuccess; --c) {
     if (max_net_nodes <= cls.nmax[c - 1]) continue;
     const int nmax = std::min(cls.nmax[c], max_net_nodes);
-    err = launch_shape(tn.shape[c - 1], job, L(c), counters + c, work + c, nmax, di.sms,
-                       next_stream());
+    cudaStream_t st = next_stream();
+    err = launch_shape(tn.shape[c - 1], job, L(c), counters + c, work + c, nmax, di.sms, chained,
+                       st);
   }
   if (err == cudaSuccess) {
-    rc_small_kernel<<<small_ctas(cap, di.sms), 32, 0, next_stream()>>>(
-        job, L(0), counters + 0, cap, max_net_nodes, status);
-    count_launch();
-    err = cudaGetLastError();
+    cudaStream_t st = next_stream();
+    err = chain_launch(rc_small_kernel, small_ctas(cap, di.sms), 32, 0, 1, chained, st, job, L(0),
+                       counters + 0, cap, max_net_nodes, status);
   }
   // join (also after a failed launch, so a capture is never left unjoined)
   for (int i = 0; i < nside; ++i) {

@@ -17,7 +17,7 @@
 //
 // Why four lanes: a net of nine nodes keeps nine lanes of a warp busy when
 // the warp takes one net, and its sweeps are O(n) shuffles each (337 us for
-// 250,000 nets of 2..16 nodes with sinks; now 141 us).  One lane per net
+// 250,000 nets of 2..16 nodes with sinks; now 152 us).  One lane per net
 // runs fewer instructions but leaves six warps per SM, too few to hide the
 // serial sweeps (261 us).  What bounds it: the load/store unit (about 13
 // shared-memory and L1 wavefronts per node, 75% busy; 16-byte cells packed
@@ -283,4 +283,5 @@ __global__ void __launch_bounds__(32) rc_small_kernel(RcJob job, const int* list
     }
     __syncwarp();  // sorted is written again
   }
+  chain_end();
 }
