@@ -133,6 +133,75 @@ __device__ Lut timing_lut(const G& G_, int t, int which, int irf, int orf) {
   return Lut{m.x, m.y, m.z, m.w};
 }
 
+// The query of a table staged on chip whose load is known before its slew.
+// Everything that does not need the slew -- the load's segment and its
+// distances -- is prepared while the slew's pin is waited for, and what is
+// left runs without branches: the slew's segment by counting (all axis
+// entries in flight at once), four table entries, three interpolations.
+// The operations and their order are lut_eval's, so the value is the same
+// bit for bit.  Only tables with the slew on their first axis and 2..8
+// entries per axis take it (the generated and the bundled libraries' 7x7
+// tables); others go through timing_value.  With both of a cell arc's
+// tables interleaved this is about 500 cycles on the critical path of every
+// gate; two calls of timing_value, each with two binary searches of generic
+// loads and three four-way branches, were 3500.
+constexpr int kPrepAxis = 8;
+struct Prep {
+  int ax, tb;    // s_lut index of the slew axis, and of the entry (0, load segment's start)
+  int n1, n2;    // n1 = 0: not prepared
+  float dx, d2;  // load - its reference end, the load segment's length
+  int pick;      // 0, 1: extrapolate from the lower, the upper end; 2, 3: exactly that end's value
+};
+
+__device__ __forceinline__ Prep prep_lut(const Lut& m, int lut_smem, float load) {
+  extern __shared__ float s_lut[];
+  Prep p{0, 0, 0, 0, 0.0f, 1.0f, 0};
+  if (m.var != 0 || m.n1 < 2 || m.n1 > kPrepAxis || m.n2 < 2 || m.n2 > kPrepAxis || m.off < 0 ||
+      m.off + m.n1 + m.n2 + m.n1 * m.n2 > lut_smem || !(fabsf(load) < 3.402823466e+38f))
+    return p;
+  const float* i2 = s_lut + m.off + m.n1;
+  int below = 0;
+#pragma unroll
+  for (int i = 0; i < kPrepAxis; ++i) below += i < m.n2 && i2[min(i, m.n2 - 1)] < load;
+  const int a2 = max(1, min(below, m.n2 - 1));
+  const float x1 = i2[a2 - 1], x2 = i2[a2];
+  p.ax = m.off;
+  p.tb = m.off + m.n1 + m.n2 + a2 - 1;
+  p.n1 = m.n1;
+  p.n2 = m.n2;
+  p.dx = __fsub_rn(load, load > x2 ? x2 : x1);
+  p.d2 = __fsub_rn(x2, x1);
+  p.pick = load == x1 ? 2 : (load == x2 ? 3 : (load > x2 ? 1 : 0));
+  return p;
+}
+
+// interpolate() between (x1, y1) and (x2, y2) at x, in selects: below x1,
+// y1 - (x1 - x) * slope is y1 + (x - x1) * slope bit for bit.
+__device__ __forceinline__ float interp_sel(float x, float x1, float x2, float y1, float y2) {
+  const float slope = __fdiv_rn(__fsub_rn(y2, y1), __fsub_rn(x2, x1));
+  const bool above = x > x2;
+  float y = __fadd_rn(above ? y2 : y1, __fmul_rn(__fsub_rn(x, above ? x2 : x1), slope));
+  y = x == x1 ? y1 : (x == x2 ? y2 : y);
+  return fabsf(x) >= 3.402823466e+38f ? x : y;
+}
+
+__device__ __forceinline__ float prep_value(const Prep& p, float slew) {
+  extern __shared__ float s_lut[];
+  const float* i1 = s_lut + p.ax;
+  int below = 0;
+#pragma unroll
+  for (int i = 0; i < kPrepAxis; ++i) below += i < p.n1 && i1[min(i, p.n1 - 1)] < slew;
+  const int a1 = max(1, min(below, p.n1 - 1));
+  const float x1 = i1[a1 - 1], x2 = i1[a1];
+  const float* t1 = s_lut + p.tb + (a1 - 1) * p.n2;
+  const float* t2 = t1 + p.n2;
+  const float lo = interp_sel(slew, x1, x2, t1[0], t2[0]);
+  const float hi = interp_sel(slew, x1, x2, t1[1], t2[1]);
+  const float y = __fadd_rn((p.pick & 1) ? hi : lo,
+                            __fmul_rn(p.dx, __fdiv_rn(__fsub_rn(hi, lo), p.d2)));
+  return p.pick >= 2 ? ((p.pick & 1) ? hi : lo) : y;
+}
+
 // The query itself; (a, b) = (slew, load) for delay and slew, (related
 // slew, constrained slew) for constraint.
 // Where the tables are read: the staged copy (floats [0, n)) for a table
@@ -143,7 +212,7 @@ struct LutSrc {
   const float* gmem;
 };
 
-__device__ float timing_value(const LutSrc& src, const Lut& m, float a, float b) {
+__device__ __noinline__ float timing_value(const LutSrc& src, const Lut& m, float a, float b) {
   if (m.n1 < 0) return nanf("");
   const bool staged = m.off >= 0 && m.off + m.n1 + m.n2 + m.n1 * m.n2 <= src.n;
   const float* lutd = staged ? src.smem : src.gmem;
@@ -175,51 +244,68 @@ __device__ __forceinline__ float ld_relaxed(const float* p) {
   return v;
 }
 
+__device__ __forceinline__ float4 ld_relaxed4(const float* p) {
+  float4 v;
+  asm volatile("ld.relaxed.gpu.global.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+
 __device__ __forceinline__ void st_relaxed4(float* p, float a, float b, float c, float d) {
   asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b),
                "f"(c), "f"(d)
                : "memory");
 }
 
-// Bounded wait until *p holds a computed value, returned in out; false
-// when this or another wait gave up.  Each poll is one L2 round trip: the
-// abort flag and the clock are read on every 8th poll only, and no poll
-// sleeps, since a sleeping warp sees a new value only after it wakes.
-__device__ bool wait_value(const float* p, float& out, GridCtl* c) {
-  out = ld_relaxed(p);
-  if (__float_as_uint(out) != kPending) return true;
+// Bounded wait of a whole warp: load() reads a lane's words again, pending()
+// says whether one of them is still not computed.  False (in every lane)
+// when this or another wait gave up.  The lanes wait together: lanes that
+// went on alone as their values came in would run the code after the wait
+// one group after another, the last to come behind all others.  Each poll
+// is one L2 round trip: the abort flag and the clock are read on every 8th
+// poll only, and no poll sleeps, since a sleeping warp sees a new value
+// only after it wakes.
+template <class LoadF, class PendF>
+__device__ __forceinline__ bool wait_warp(LoadF load, PendF pending, GridCtl* c) {
+  load();
+  if (!__any_sync(FULL, pending())) return true;
   const unsigned long long t0 = gtime();
   for (int k = 0;; ++k) {
-    out = ld_relaxed(p);
-    if (__float_as_uint(out) != kPending) return true;
+    if (pending()) load();
+    if (!__any_sync(FULL, pending())) return true;
     if ((k & 7) != 7) continue;
-    if (*(volatile int*)&c->abort) return false;
-    if (gtime() - t0 > kGridWaitNs) {
+    const bool late = gtime() - t0 > kGridWaitNs;
+    if (late) {
       atomicExch(&c->abort, 1);
       atomicCAS(&c->status, 0, (int)OTG_ERR_TIMEOUT);
-      return false;
     }
+    if (__any_sync(FULL, late || *(volatile int*)&c->abort)) return false;
   }
 }
 
-// wait_value for two words at once: both loads in flight per poll.
-__device__ bool wait_values(const float* p, const float* q, float& x, float& y, GridCtl* c) {
-  x = ld_relaxed(p);
-  y = ld_relaxed(q);
-  if (__float_as_uint(x) != kPending && __float_as_uint(y) != kPending) return true;
-  const unsigned long long t0 = gtime();
-  for (int k = 0;; ++k) {
-    if (__float_as_uint(x) == kPending) x = ld_relaxed(p);
-    if (__float_as_uint(y) == kPending) y = ld_relaxed(q);
-    if (__float_as_uint(x) != kPending && __float_as_uint(y) != kPending) return true;
-    if ((k & 7) != 7) continue;
-    if (*(volatile int*)&c->abort) return false;
-    if (gtime() - t0 > kGridWaitNs) {
-      atomicExch(&c->abort, 1);
-      atomicCAS(&c->status, 0, (int)OTG_ERR_TIMEOUT);
-      return false;
-    }
-  }
+__device__ __forceinline__ bool is_pending(float x) { return __float_as_uint(x) == kPending; }
+
+// Until *p and *q hold computed values in the lanes that are `on`.
+__device__ __forceinline__ bool wait_values(bool on, const float* p, const float* q, float& x,
+                                            float& y, GridCtl* c) {
+  x = y = 0.0f;
+  return wait_warp(
+      [&] {
+        if (!on) return;
+        x = ld_relaxed(p);
+        y = ld_relaxed(q);
+      },
+      [&] { return is_pending(x) || is_pending(y); }, c);
+}
+__device__ __forceinline__ bool wait_value(bool on, const float* p, float& x, GridCtl* c) {
+  x = 0.0f;
+  return wait_warp(
+      [&] {
+        if (on) x = ld_relaxed(p);
+      },
+      [&] { return is_pending(x); }, c);
 }
 
 // Order-free relax of Pin::_relax_slew/_relax_at (MIN keeps the smallest,
@@ -250,16 +336,19 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
     sl = __ldg(g.pi_slew + 4 * v + c_out);
     a = __ldg(g.pi_at + 4 * v + c_out);
   }
-  bool ok = true;
-  for (int j = lane; j < nitems; j += 32) {
-    const int arc = __ldg(g.fanin + f0 + (j >> 3));
-    const int u = __ldg(g.arc_from + arc);
-    const int kind = __ldg(g.arc_kind + arc);
+  for (int j0 = 0; j0 < nitems; j0 += 32) {
+    const int j = j0 + lane;
+    const bool on = j < nitems;  // the last pass may leave lanes without an arc
+    const int arc = on ? __ldg(g.fanin + f0 + (j >> 3)) : 0;
+    const int u = on ? __ldg(g.arc_from + arc) : 0;
+    const int kind = on ? __ldg(g.arc_kind + arc) : 0;
     float d = nanf(""), so = nanf(""), imp = nanf("");
     Lut ls = no_lut(), ld = no_lut();
+    Prep ps, pd;
+    ps.n1 = pd.n1 = 0;
     float load = 0.0f;
     int s = -1;
-    if (kind == 0) {
+    if (kind == 0 && on) {
       s = frf == trf ? rc_slot(G_, arc) : -1;
       if (s >= 0) {
         imp = __ldg(G_.rc.impulse + 4 * (size_t)s + c_out);
@@ -283,6 +372,8 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
       const int net = __ldg(g.arc_net + arc);
       if (net >= 0 && t >= 0)
         load = __ldg(G_.rc.load + 4 * (size_t)__ldg(G_.rc.nodes_start + net) + c_out);
+      ps = prep_lut(ls, lutd.n, load);
+      pd = prep_lut(ld, lutd.n, load);
       const int uf0 = __ldg(g.fanin_start + u);
       if (__ldg(g.fanin_start + u + 1) - uf0 == 1) {
         const int a0 = __ldg(g.fanin + uf0);
@@ -301,10 +392,8 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
       }
     }
     float si, fa;
-    if (!wait_values(slew + 4 * src + 2 * el + frf, at + 4 * src + 2 * el + frf, si, fa, ctl)) {
-      ok = false;
-      break;
-    }
+    if (!wait_values(on, slew + 4 * src + 2 * el + frf, at + 4 * src + 2 * el + frf, si, fa, ctl))
+      return false;
     if (thru) {
       float so_u = nanf(""), at_u = nanf("");
       if (t_s >= 0 && !none(si)) {
@@ -321,18 +410,21 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
         const float r = sqrtf(__fadd_rn(__fmul_rn(si, si), imp));
         so = si < 0.0f ? -r : r;
       }
-    } else if (!none(si)) {
+    } else if (none(si)) {
+      d = nanf("");
+    } else if (ps.n1 && pd.n1) {
+      so = prep_value(ps, si);
+      d = prep_value(pd, si);
+    } else {
       so = timing_value(lutd, ls, si, load);
       d = timing_value(lutd, ld, si, load);
-    } else {
-      d = nanf("");
     }
+    if (!on) continue;
     arc_delay[8 * (size_t)arc + (j & 7)] = d;
     sl = relax_fwd(el, sl, so);
     if (!none(fa) && !none(d)) a = relax_fwd(el, a, __fadd_rn(d, fa));
   }
-  ok = __all_sync(FULL, ok);
-  if (!ok) return false;
+  __syncwarp();
   // lanes sharing (el, trf) differ in bits 1, 3 and 4
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -359,42 +451,102 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
   // timing tests constrained at v (Test::_fprop_rat): lane j of a pass takes
   // test j/4 and output corner j%4
   const int t0 = __ldg(g.test_start + v), ntest = 4 * (__ldg(g.test_start + v + 1) - t0);
-  for (int j = lane; j < ntest; j += 32) {
-    const int test = __ldg(g.test_of_pin + t0 + (j >> 2));
-    const int arc = __ldg(g.test_arc + test), u = __ldg(g.arc_from + arc);
+  for (int j0 = 0; j0 < ntest; j0 += 32) {
+    const int j = j0 + lane;
+    const bool on = j < ntest;
+    const int test = on ? __ldg(g.test_of_pin + t0 + (j >> 2)) : 0;
+    const int arc = on ? __ldg(g.test_arc + test) : 0, u = on ? __ldg(g.arc_from + arc) : 0;
     const int tel = (j >> 1) & 1, rf = j & 1;
-    const int t = __ldg(g.arc_timing + 2 * arc + tel);
+    const int t = on ? __ldg(g.arc_timing + 2 * arc + tel) : -1;
     float val = nanf("");
-    if (!none(g.period) && t >= 0) {
-      const int edge = __ldg(g.timing + 9 * t + 1);
-      const int fel = tel == MIN_ ? MAX_ : MIN_;
-      const int rrf = edge == 1 ? RISE_ : FALL_;
-      const float csl = slc[2 * tel + rf];
-      if (!(rrf == FALL_ && edge != 2) && !none(csl)) {
-        const Lut lc = timing_lut(G_, t, 2, rrf, rf);
-        float rat_at, rsl;
-        if (!wait_values(at + 4 * u + 2 * fel + rrf, slew + 4 * u + 2 * fel + rrf, rat_at, rsl,
-                         ctl)) {
-          ok = false;
-          break;
-        }
-        if (!none(rat_at) && !none(rsl)) {
-          const float related = tel == MIN_ ? rat_at : __fadd_rn(rat_at, g.period);
-          const float cons = timing_value(lutd, lc, rsl, csl);
-          if (!none(cons))
-            val = tel == MIN_ ? __fadd_rn(cons, related) : __fsub_rn(related, cons);
-        }
-      }
+    const int edge = t >= 0 ? __ldg(g.timing + 9 * t + 1) : 0;
+    const int fel = tel == MIN_ ? MAX_ : MIN_;
+    const int rrf = edge == 1 ? RISE_ : FALL_;
+    const float csl = slc[2 * tel + rf];
+    const bool asks =
+        t >= 0 && !none(g.period) && !(rrf == FALL_ && edge != 2) && !none(csl);
+    const Lut lc = asks ? timing_lut(G_, t, 2, rrf, rf) : no_lut();
+    float rat_at, rsl;
+    if (!wait_values(asks, at + 4 * u + 2 * fel + rrf, slew + 4 * u + 2 * fel + rrf, rat_at, rsl,
+                     ctl))
+      return false;
+    if (asks && !none(rat_at) && !none(rsl)) {
+      const float related = tel == MIN_ ? rat_at : __fadd_rn(rat_at, g.period);
+      const float cons = timing_value(lutd, lc, rsl, csl);
+      if (!none(cons)) val = tel == MIN_ ? __fadd_rn(cons, related) : __fsub_rn(related, cons);
     }
-    test_rat[4 * (size_t)test + (j & 3)] = val;
+    if (on) test_rat[4 * (size_t)test + (j & 3)] = val;
   }
-  return __all_sync(FULL, ok);
+  return true;
+}
+
+// The net arcs among a driver's many fanouts, kNetArcs to a lane at a time,
+// all four corners of an arc at once (a net arc only relates equal
+// transitions).  Eight lanes an arc, as below, hold four arcs in flight: a
+// clock driver of 12,000 sinks then takes 3000 rounds of three dependent
+// loads, 3.9 ms of a 4.9 ms propagation of 240,000 gates.  *cells: some
+// other arc is among them.
+constexpr int kNetArcs = 4;
+__device__ __forceinline__ bool bprop_net_arcs(const otg_prop_graph& g, int o0, int num, int lane,
+                                               const float* rat, const float* arc_delay,
+                                               float (&r)[4], bool* cells, GridCtl* ctl) {
+  *cells = false;
+  for (int j0 = 0; j0 < num; j0 += 32 * kNetArcs) {
+    int arc[kNetArcs], w[kNetArcs];
+    float4 lo[kNetArcs], hi[kNetArcs], x[kNetArcs];
+#pragma unroll
+    for (int u = 0; u < kNetArcs; ++u) {
+      const int j = j0 + 32 * u + lane;
+      arc[u] = j < num ? __ldg(g.fanout + o0 + j) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < kNetArcs; ++u) {
+      w[u] = -1;
+      x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (arc[u] < 0) continue;
+      if (__ldg(g.arc_kind + arc[u]) == 0) w[u] = __ldg(g.arc_to + arc[u]);
+      else *cells = true;
+      const float4* d = reinterpret_cast<const float4*>(arc_delay) + 2 * (size_t)arc[u];
+      lo[u] = __ldcg(d);
+      hi[u] = __ldcg(d + 1);
+    }
+    auto pend = [](const float4& v) {
+      return is_pending(v.x) || is_pending(v.y) || is_pending(v.z) || is_pending(v.w);
+    };
+    const bool there = wait_warp(
+        [&] {
+#pragma unroll
+          for (int u = 0; u < kNetArcs; ++u)
+            if (w[u] >= 0) x[u] = ld_relaxed4(rat + 4 * w[u]);
+        },
+        [&] {
+          bool p = false;
+#pragma unroll
+          for (int u = 0; u < kNetArcs; ++u) p |= pend(x[u]);
+          return p;
+        },
+        ctl);
+    if (!there) return false;
+#pragma unroll
+    for (int u = 0; u < kNetArcs; ++u) {
+      if (w[u] < 0) continue;
+      const float wr[4] = {x[u].x, x[u].y, x[u].z, x[u].w};
+      const float dl[4] = {lo[u].x, lo[u].w, hi[u].x, hi[u].w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (!none(wr[c]) && !none(dl[c]))
+          r[c] = relax_bwd(c >> 1, r[c], __fsub_rn(wr[c], dl[c]));
+    }
+  }
+  *cells = __any_sync(FULL, *cells);
+  return true;
 }
 
 // Backward at pin v (one warp): Timer::_bprop_rat and the slack.  Lanes
 // first take the tests constrained at v (4 corners each), then the fanout
 // arcs (8 combinations each); every candidate lands in a 4-corner register
-// set reduced over the whole warp.
+// set reduced over the whole warp.  The net arcs of a pin with more fanouts
+// than one pass takes go through bprop_net_arcs.
 __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float* rat, float* slack,
                            const float* arc_delay, const float* test_rat, GridCtl* ctl) {
   const otg_prop_graph& g = G_.g;
@@ -402,23 +554,33 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
 #pragma unroll
   for (int c = 0; c < 4; ++c) r[c] = lane == 0 ? __ldg(g.po_rat + 4 * v + c) : nanf("");
   const int t0 = __ldg(g.test_start + v), ntest = 4 * (__ldg(g.test_start + v + 1) - t0);
-  const int o0 = __ldg(g.fanout_start + v), nitems = ntest + 8 * (__ldg(g.fanout_start + v + 1) - o0);
-  bool ok = true;
-  for (int j = lane; j < nitems; j += 32) {
+  const int o0 = __ldg(g.fanout_start + v), nout = __ldg(g.fanout_start + v + 1) - o0;
+  int nitems = ntest + 8 * nout;
+  const bool many = nout > 4;
+  if (many) {
+    bool cells;
+    if (!bprop_net_arcs(g, o0, nout, lane, rat, arc_delay, r, &cells, ctl)) return false;
+    if (!cells) nitems = ntest;
+  }
+  for (int j0 = 0; j0 < nitems; j0 += 32) {
+    const int j = j0 + lane;
     int tc = 0;  // target corner
     float cand = nanf("");
+    int mode = 0;  // 0 none, 1 propagation, 2 MIN constraint, 3 MAX constraint
+    int wc = 0, w = 0, el = 0, frf = 0, trf = 0;
+    float dl = nanf(""), a = nanf(""), wa = nanf("");
     if (j < ntest) {
       tc = j & 3;
       cand = __ldcg(test_rat + 4 * (size_t)__ldg(g.test_of_pin + t0 + (j >> 2)) + tc);
-    } else {
+    } else if (j < nitems) {
       const int jj = j - ntest;
-      const int arc = __ldg(g.fanout + o0 + (jj >> 3)), w = __ldg(g.arc_to + arc);
-      const int el = (jj >> 2) & 1, frf = (jj >> 1) & 1, trf = jj & 1;
-      const int kind = __ldg(g.arc_kind + arc);
-      const float* d = arc_delay + 8 * (size_t)arc;
-      int mode = 0;  // 0 none, 1 propagation, 2 MIN constraint, 3 MAX constraint
-      if (kind == 0) {
-        mode = frf == trf ? 1 : 0;
+      const int arc = __ldg(g.fanout + o0 + (jj >> 3));
+      w = __ldg(g.arc_to + arc);
+      el = (jj >> 2) & 1;
+      frf = (jj >> 1) & 1;
+      trf = jj & 1;
+      if (__ldg(g.arc_kind + arc) == 0) {
+        mode = frf == trf && !many ? 1 : 0;
       } else {
         const int t = __ldg(g.arc_timing + 2 * arc + el);
         if (t >= 0) {
@@ -427,42 +589,34 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
           else if (transition_defined(tr, frf, trf)) mode = el == MIN_ ? 2 : 3;
         }
       }
-      if (mode != 0) {
-        // the fanout's required time this combination reads
-        const int wc = mode == 1 ? 2 * el + trf : (mode == 2 ? trf : 2 + trf);
-        // arc delays and arrival times are final since the forward pass, so
-        // they are loaded before the wait and arrive during it
-        float dl = nanf(""), a = nanf(""), wa = nanf("");
-        if (mode == 1) {
-          dl = __ldcg(d + 4 * el + 2 * frf + trf);
-        } else {
-          const int ael = mode == 2 ? MAX_ : MIN_, wel = mode == 2 ? MIN_ : MAX_;
-          a = __ldcg(at + 4 * v + 2 * ael + frf);
-          wa = __ldcg(at + 4 * w + 2 * wel + trf);
-        }
-        float wr;
-        if (!wait_value(rat + 4 * w + wc, wr, ctl)) {
-          ok = false;
-          break;
-        }
-        if (mode == 1) {
-          tc = 2 * el + frf;
-          if (!none(wr) && !none(dl)) cand = __fsub_rn(wr, dl);
-        } else if (mode == 2) {  // hold-like: w's MIN slack moves v's MAX rat
-          tc = 2 * MAX_ + frf;
-          if (!none(a) && !none(wa) && !none(wr)) cand = __fadd_rn(a, __fsub_rn(wa, wr));
-        } else {  // setup-like: w's MAX slack moves v's MIN rat
-          tc = 2 * MIN_ + frf;
-          if (!none(a) && !none(wa) && !none(wr)) cand = __fsub_rn(a, __fsub_rn(wr, wa));
-        }
+      // the fanout's required time this combination reads; arc delays and
+      // arrival times are final since the forward pass, so they are loaded
+      // before the wait and arrive during it
+      wc = mode == 1 ? 2 * el + trf : (mode == 2 ? trf : 2 + trf);
+      if (mode == 1) {
+        dl = __ldcg(arc_delay + 8 * (size_t)arc + 4 * el + 2 * frf + trf);
+      } else if (mode != 0) {
+        const int ael = mode == 2 ? MAX_ : MIN_, wel = mode == 2 ? MIN_ : MAX_;
+        a = __ldcg(at + 4 * v + 2 * ael + frf);
+        wa = __ldcg(at + 4 * w + 2 * wel + trf);
       }
+    }
+    float wr;
+    if (!wait_value(mode != 0, rat + 4 * w + wc, wr, ctl)) return false;
+    if (mode == 1) {
+      tc = 2 * el + frf;
+      if (!none(wr) && !none(dl)) cand = __fsub_rn(wr, dl);
+    } else if (mode == 2) {  // hold-like: w's MIN slack moves v's MAX rat
+      tc = 2 * MAX_ + frf;
+      if (!none(a) && !none(wa) && !none(wr)) cand = __fadd_rn(a, __fsub_rn(wa, wr));
+    } else if (mode == 3) {  // setup-like: w's MAX slack moves v's MIN rat
+      tc = 2 * MIN_ + frf;
+      if (!none(a) && !none(wa) && !none(wr)) cand = __fsub_rn(a, __fsub_rn(wr, wa));
     }
 #pragma unroll
     for (int c = 0; c < 4; ++c)
       if (c == tc) r[c] = relax_bwd(c >> 1, r[c], cand);
   }
-  ok = __all_sync(FULL, ok);
-  if (!ok) return false;
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
@@ -546,8 +700,9 @@ __global__ void __launch_bounds__(256) prop_kernel(G G_, const int* order, const
 size_t align256p(size_t x) { return (x + 255) & ~(size_t)255; }
 
 // Tables up to this many floats are staged in shared memory (40 KB per
-// CTA keeps five 256-thread CTAs per SM; a library with three drive
-// strengths of its combinational cells takes about 33 KB).
+// CTA leaves room for the four 256-thread CTAs per SM that the registers
+// allow; a library with three drive strengths of its combinational cells
+// takes about 33 KB).
 constexpr int kLutSmemFloats = 10240;
 
 struct PropDev {
