@@ -44,6 +44,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 
 #include "../../include/otg.h"
 #include "otg_internal.cuh"
@@ -133,75 +134,6 @@ __device__ Lut timing_lut(const G& G_, int t, int which, int irf, int orf) {
   return Lut{m.x, m.y, m.z, m.w};
 }
 
-// The query of a table staged on chip whose load is known before its slew.
-// Everything that does not need the slew -- the load's segment and its
-// distances -- is prepared while the slew's pin is waited for, and what is
-// left runs without branches: the slew's segment by counting (all axis
-// entries in flight at once), four table entries, three interpolations.
-// The operations and their order are lut_eval's, so the value is the same
-// bit for bit.  Only tables with the slew on their first axis and 2..8
-// entries per axis take it (the generated and the bundled libraries' 7x7
-// tables); others go through timing_value.  With both of a cell arc's
-// tables interleaved this is about 500 cycles on the critical path of every
-// gate; two calls of timing_value, each with two binary searches of generic
-// loads and three four-way branches, were 3500.
-constexpr int kPrepAxis = 8;
-struct Prep {
-  int ax, tb;    // s_lut index of the slew axis, and of the entry (0, load segment's start)
-  int n1, n2;    // n1 = 0: not prepared
-  float dx, d2;  // load - its reference end, the load segment's length
-  int pick;      // 0, 1: extrapolate from the lower, the upper end; 2, 3: exactly that end's value
-};
-
-__device__ __forceinline__ Prep prep_lut(const Lut& m, int lut_smem, float load) {
-  extern __shared__ float s_lut[];
-  Prep p{0, 0, 0, 0, 0.0f, 1.0f, 0};
-  if (m.var != 0 || m.n1 < 2 || m.n1 > kPrepAxis || m.n2 < 2 || m.n2 > kPrepAxis || m.off < 0 ||
-      m.off + m.n1 + m.n2 + m.n1 * m.n2 > lut_smem || !(fabsf(load) < 3.402823466e+38f))
-    return p;
-  const float* i2 = s_lut + m.off + m.n1;
-  int below = 0;
-#pragma unroll
-  for (int i = 0; i < kPrepAxis; ++i) below += i < m.n2 && i2[min(i, m.n2 - 1)] < load;
-  const int a2 = max(1, min(below, m.n2 - 1));
-  const float x1 = i2[a2 - 1], x2 = i2[a2];
-  p.ax = m.off;
-  p.tb = m.off + m.n1 + m.n2 + a2 - 1;
-  p.n1 = m.n1;
-  p.n2 = m.n2;
-  p.dx = __fsub_rn(load, load > x2 ? x2 : x1);
-  p.d2 = __fsub_rn(x2, x1);
-  p.pick = load == x1 ? 2 : (load == x2 ? 3 : (load > x2 ? 1 : 0));
-  return p;
-}
-
-// interpolate() between (x1, y1) and (x2, y2) at x, in selects: below x1,
-// y1 - (x1 - x) * slope is y1 + (x - x1) * slope bit for bit.
-__device__ __forceinline__ float interp_sel(float x, float x1, float x2, float y1, float y2) {
-  const float slope = __fdiv_rn(__fsub_rn(y2, y1), __fsub_rn(x2, x1));
-  const bool above = x > x2;
-  float y = __fadd_rn(above ? y2 : y1, __fmul_rn(__fsub_rn(x, above ? x2 : x1), slope));
-  y = x == x1 ? y1 : (x == x2 ? y2 : y);
-  return fabsf(x) >= 3.402823466e+38f ? x : y;
-}
-
-__device__ __forceinline__ float prep_value(const Prep& p, float slew) {
-  extern __shared__ float s_lut[];
-  const float* i1 = s_lut + p.ax;
-  int below = 0;
-#pragma unroll
-  for (int i = 0; i < kPrepAxis; ++i) below += i < p.n1 && i1[min(i, p.n1 - 1)] < slew;
-  const int a1 = max(1, min(below, p.n1 - 1));
-  const float x1 = i1[a1 - 1], x2 = i1[a1];
-  const float* t1 = s_lut + p.tb + (a1 - 1) * p.n2;
-  const float* t2 = t1 + p.n2;
-  const float lo = interp_sel(slew, x1, x2, t1[0], t2[0]);
-  const float hi = interp_sel(slew, x1, x2, t1[1], t2[1]);
-  const float y = __fadd_rn((p.pick & 1) ? hi : lo,
-                            __fmul_rn(p.dx, __fdiv_rn(__fsub_rn(hi, lo), p.d2)));
-  return p.pick >= 2 ? ((p.pick & 1) ? hi : lo) : y;
-}
-
 // The query itself; (a, b) = (slew, load) for delay and slew, (related
 // slew, constrained slew) for constraint.
 // Where the tables are read: the staged copy (floats [0, n)) for a table
@@ -222,6 +154,105 @@ __device__ __noinline__ float timing_value(const LutSrc& src, const Lut& m, floa
   }
   // var 0: (slew | related) first; var 1: (load | constrained) first
   return m.var == 0 ? lut_eval(m, lutd, a, b) : lut_eval(m, lutd, b, a);
+}
+
+// A cell arc's table at a load that is known before the slew: reduced,
+// while the slew's pin is waited for, to its values along the slew axis at
+// that load, kept in shared memory; what is left for after the wait is the
+// slew's segment (by counting, all axis entries in flight at once) and one
+// interpolation.  In exact arithmetic the same bilinear form as lut_eval's,
+// whichever axis comes first.  Slew axes of up to kPrepAxis entries; others
+// go through timing_value.  After the wait an arc's two tables take about
+// 250 cycles of every gate on a path; interpolating both axes there took
+// 1700 (six divisions, each with its own branch), and two calls of
+// timing_value 3500.
+constexpr int kPrepAxis = 8, kPropT = 256;
+// floats of shared memory: the values of two tables per thread, and, where
+// the library is not staged, their slew axes
+constexpr int kPrepFloats = 2 * kPrepAxis * kPropT;
+struct Prep {
+  int n;           // entries of the slew axis; 0: not prepared
+  int ax, stride;  // the axis in shared memory: ax, ax + stride, ...
+  int at;          // the values: at, at + kPropT, ...
+};
+
+// which: 0, 1 of the thread's tables; prep0: where the prepared values start.
+__device__ __forceinline__ Prep prep_lut(const LutSrc& src, const Lut& m, float load, int which,
+                                         int prep0) {
+  extern __shared__ float s_lut[];
+  Prep p{0, 0, 1, prep0 + which * kPrepAxis * kPropT + (int)threadIdx.x};
+  const int ns = m.var == 0 ? m.n1 : m.n2, nl = m.var == 0 ? m.n2 : m.n1;
+  if (m.n1 < 1 || m.n2 < 1 || m.var < 0 || ns > kPrepAxis || !(fabsf(load) < 3.402823466e+38f))
+    return p;
+  const bool staged = m.off >= 0 && m.off + m.n1 + m.n2 + m.n1 * m.n2 <= src.n;
+  if (!staged && src.n > 0) return p;  // no room was left for its axis
+  const float* i1 = (staged ? src.smem : src.gmem) + m.off;
+  const float* i2 = i1 + m.n1;
+  const float* e = i2 + m.n2;  // entry of the load segment's start, first slew
+  const float* lax = m.var == 0 ? i2 : i1;
+  const int ds = m.var == 0 ? m.n2 : 1, dl = m.var == 0 ? 1 : m.n2;  // steps along slew, load
+  float f = 0.0f;
+  if (nl > 1) {
+    const int a = max(1, min(lower_bound(lax, nl, load), nl - 1));
+    f = __fdiv_rn(__fsub_rn(load, lax[a - 1]), __fsub_rn(lax[a], lax[a - 1]));
+    e += (a - 1) * dl;
+  }
+  const int next = nl > 1 ? dl : 0;
+#pragma unroll
+  for (int i = 0; i < kPrepAxis; ++i)
+    if (i < ns) {
+      const float x = e[i * ds];
+      s_lut[p.at + i * kPropT] = __fmaf_rn(f, __fsub_rn(e[i * ds + next], x), x);
+    }
+  if (staged) {
+    p.ax = m.off + (m.var == 0 ? 0 : m.n1);
+  } else {
+    const float* sax = m.var == 0 ? i1 : i2;
+    p.ax = p.at + kPrepFloats;
+    p.stride = kPropT;
+#pragma unroll
+    for (int i = 0; i < kPrepAxis; ++i)
+      if (i < ns) s_lut[p.ax + i * kPropT] = sax[i];
+  }
+  p.n = ns;
+  return p;
+}
+
+// Whether two prepared tables have the same slew axis.
+__device__ __forceinline__ bool same_axis(const Prep& a, const Prep& b) {
+  extern __shared__ float s_lut[];
+  bool same = a.n == b.n;
+#pragma unroll
+  for (int i = 0; i < kPrepAxis; ++i) {
+    const int k = min(i, max(min(a.n, b.n) - 1, 0));
+    same = same & (s_lut[a.ax + k * a.stride] == s_lut[b.ax + k * b.stride]);
+  }
+  return same;
+}
+
+// The slew's segment on p's axis (its start, 0-based) and how far along it
+// the slew is.  No branch depends on p: half of a gate's lanes have no
+// table (the other split's, or the transitions the arc does not make), and
+// branching around them cost 1000 cycles per gate.
+__device__ __forceinline__ void prep_segment(const Prep& p, float slew, int& seg, float& t) {
+  extern __shared__ float s_lut[];
+  const int last = max(p.n - 1, 0);
+  int below = 0;
+#pragma unroll
+  for (int i = 0; i < kPrepAxis; ++i)
+    below += (int)(i < p.n) & (int)(s_lut[p.ax + min(i, last) * p.stride] < slew);
+  seg = max(0, min(below, last) - 1);
+  const float x1 = s_lut[p.ax + seg * p.stride];
+  const float x2 = s_lut[p.ax + min(seg + 1, last) * p.stride];
+  t = __fdiv_rn(p.n > 1 ? __fsub_rn(slew, x1) : 0.0f, p.n > 1 ? __fsub_rn(x2, x1) : 1.0f);
+}
+
+__device__ __forceinline__ float prep_value(const Prep& p, int seg, float t) {
+  extern __shared__ float s_lut[];
+  const float lo = s_lut[p.at + seg * kPropT];
+  const float hi = s_lut[p.at + (p.n > 1 ? seg + 1 : 0) * kPropT];
+  const float y = __fmaf_rn(t, __fsub_rn(hi, lo), lo);
+  return p.n > 0 ? y : nanf("");
 }
 
 // RC node of a net arc's sink (arc_node: its local id in the net) as a
@@ -253,6 +284,9 @@ __device__ __forceinline__ float4 ld_relaxed4(const float* p) {
   return v;
 }
 
+__device__ __forceinline__ void st_relaxed(float* p, float v) {
+  asm volatile("st.relaxed.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(v) : "memory");
+}
 __device__ __forceinline__ void st_relaxed4(float* p, float a, float b, float c, float d) {
   asm volatile("st.relaxed.gpu.global.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b),
                "f"(c), "f"(d)
@@ -318,20 +352,72 @@ __device__ __forceinline__ float relax_bwd(int el, float cur, float v) {
   return el == MIN_ ? fmaxf(cur, v) : fminf(cur, v);
 }
 
+// What a pin's forward visit reads of each fanin arc, packed by the fill so
+// that a visit follows one load instead of a chain of nine (fanin, arc,
+// input pin, its net arc, net, node, slot): x the pin to wait on, y the BFS
+// slot of the sink whose Elmore values the arc or its input pin adds (-1:
+// none), z the arc, w kNetRec for a net arc, else the load's row (-1: none).
+//
+// A cell arc out of a pin whose only fanin is a net arc (a gate's input
+// pin, without assertions) reads through it: the visit waits on the net's
+// driver and derives the input pin's slew and arrival time exactly as that
+// pin's own visit does.  The input pin still stores its own values; this
+// only shortens the chain of waits.  y is kOwnRec for the other cell arcs.
+constexpr int kNetRec = -2, kOwnRec = -2;
+constexpr int4 kNoRec = {0, -1, 0, kNetRec};
+
+__device__ __forceinline__ bool empty4(const float* p) {
+  const float x = __ldg(p), y = __ldg(p + 1), z = __ldg(p + 2), w = __ldg(p + 3);
+  return none(x) & none(y) & none(z) & none(w);
+}
+
+__device__ int4 fanin_rec(const G& G_, int arc) {
+  const otg_prop_graph& g = G_.g;
+  int4 r{__ldg(g.arc_from + arc), kOwnRec, arc, kNetRec};
+  if (__ldg(g.arc_kind + arc) == 0) {
+    r.y = rc_slot(G_, arc);
+    return r;
+  }
+  const int net = __ldg(g.arc_net + arc);
+  r.w = net >= 0 ? __ldg(G_.rc.nodes_start + net) : -1;
+  const int u = r.x, f = __ldg(g.fanin_start + u);
+  if (__ldg(g.fanin_start + u + 1) - f == 1) {
+    const int a0 = __ldg(g.fanin + f);
+    if (__ldg(g.arc_kind + a0) == 0 && empty4(g.pi_slew + 4 * u) && empty4(g.pi_at + 4 * u)) {
+      r.x = __ldg(g.arc_from + a0);
+      r.y = rc_slot(G_, a0);
+    }
+  }
+  return r;
+}
+
+// A pin a warp is about to visit: its fanin (forward) or fanout range, and
+// this lane's record or arc of the first pass.  The warp loads them while
+// it waits at the pins before.
+struct Visit {
+  int v, lo, hi;
+  int4 rec;
+};
+
 // Forward at pin v (one warp): Timer::_fprop_slew, _fprop_delay, _fprop_at
 // and _fprop_test.  Lane j of a pass takes fanin arc j/8 and the combination
 // (el, frf, trf) = bits (2, 1, 0) of j; its slew and arrival candidates go to
 // output corner (el, trf).  Returns false if a wait gave up.
-__device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, float* at,
-                           float* slew, float* rat, float* arc_delay, float* test_rat,
-                           GridCtl* ctl) {
+template <class AfterF>
+__device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const LutSrc& lutd,
+                                           int prep0, const Visit& me, int lane, float* at,
+                                           float* slew, float* rat, float* arc_delay,
+                                           float* test_rat, GridCtl* ctl, AfterF after) {
   const otg_prop_graph& g = G_.g;
+  const int v = me.v;
   const int el = (lane >> 2) & 1, frf = (lane >> 1) & 1, trf = lane & 1;
   const int c_out = 2 * el + trf;
-  const int f0 = __ldg(g.fanin_start + v), nitems = 8 * (__ldg(g.fanin_start + v + 1) - f0);
+  const int f0 = me.lo, nitems = 8 * (me.hi - f0);
   // a primary input's assertions (NaN: none) seed the lanes with frf 0 of
   // the first pass, one per output corner
   float sl = nanf(""), a = nanf("");
+  int last_arc = -1;
+  float last_d = 0.0f;
   if (lane < 8 && frf == 0) {
     sl = __ldg(g.pi_slew + 4 * v + c_out);
     a = __ldg(g.pi_at + 4 * v + c_out);
@@ -339,92 +425,77 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
   for (int j0 = 0; j0 < nitems; j0 += 32) {
     const int j = j0 + lane;
     const bool on = j < nitems;  // the last pass may leave lanes without an arc
-    const int arc = on ? __ldg(g.fanin + f0 + (j >> 3)) : 0;
-    const int u = on ? __ldg(g.arc_from + arc) : 0;
-    const int kind = on ? __ldg(g.arc_kind + arc) : 0;
+    const int4 R = j0 == 0 ? me.rec : (on ? __ldg(rec + f0 + (j >> 3)) : kNoRec);
+    const int arc = R.z;
+    const bool cell = R.w != kNetRec, thru = cell && R.y != kOwnRec;
     float d = nanf(""), so = nanf(""), imp = nanf("");
     Lut ls = no_lut(), ld = no_lut();
     Prep ps, pd;
-    ps.n1 = pd.n1 = 0;
+    ps.n = pd.n = 0;
+    bool one_axis = true, slow = false;
     float load = 0.0f;
-    int s = -1;
-    if (kind == 0 && on) {
-      s = frf == trf ? rc_slot(G_, arc) : -1;
-      if (s >= 0) {
-        imp = __ldg(G_.rc.impulse + 4 * (size_t)s + c_out);
-        d = __ldg(G_.rc.delay + 4 * (size_t)s + c_out);
-      }
+    // the sink whose Elmore delay and impulse the lane adds: a net arc's
+    // (equal transitions only), or the read-through input pin's, at (el, frf)
+    const int s = cell ? (thru ? R.y : -1) : (frf == trf ? R.y : -1);
+    if (s >= 0) {
+      const size_t row = 4 * (size_t)s + 2 * el + frf;
+      imp = __ldg(G_.rc.impulse + row);
+      d = __ldg(G_.rc.delay + row);
     }
-    // A cell arc out of a pin whose only fanin is a net arc (a gate's input
-    // pin) reads through it: the lane waits on the net's driver and derives
-    // the input pin's slew and arrival time at (el, frf) exactly as that
-    // pin's own warp does (one candidate relaxed against the assertion).
-    // The input pin still stores its own values; this only shortens the
-    // chain of waits.
-    int src = u;
-    bool thru = false;
-    float t_imp = 0.0f, t_d = nanf(""), t_psl = nanf(""), t_pat = nanf("");
-    int t_s = -1;
-    if (kind != 0) {
+    if (cell) {
       const int t = __ldg(g.arc_timing + 2 * arc + el);
       ls = timing_lut(G_, t, 1, frf, trf);
       ld = timing_lut(G_, t, 0, frf, trf);
-      const int net = __ldg(g.arc_net + arc);
-      if (net >= 0 && t >= 0)
-        load = __ldg(G_.rc.load + 4 * (size_t)__ldg(G_.rc.nodes_start + net) + c_out);
-      ps = prep_lut(ls, lutd.n, load);
-      pd = prep_lut(ld, lutd.n, load);
-      const int uf0 = __ldg(g.fanin_start + u);
-      if (__ldg(g.fanin_start + u + 1) - uf0 == 1) {
-        const int a0 = __ldg(g.fanin + uf0);
-        if (__ldg(g.arc_kind + a0) == 0) {
-          const int c_in = 2 * el + frf;
-          thru = true;
-          src = __ldg(g.arc_from + a0);
-          t_s = rc_slot(G_, a0);
-          if (t_s >= 0) {
-            t_imp = __ldg(G_.rc.impulse + 4 * (size_t)t_s + c_in);
-            t_d = __ldg(G_.rc.delay + 4 * (size_t)t_s + c_in);
-          }
-          t_psl = __ldg(g.pi_slew + 4 * u + c_in);
-          t_pat = __ldg(g.pi_at + 4 * u + c_in);
-        }
-      }
+      if (R.w >= 0 && t >= 0) load = __ldg(G_.rc.load + 4 * (size_t)R.w + c_out);
+      ps = prep_lut(lutd, ls, load, 0, prep0);
+      pd = prep_lut(lutd, ld, load, 1, prep0);
+      one_axis = ps.n == 0 || pd.n == 0 || same_axis(ps, pd);
+      slow = (ls.n1 >= 0 && ps.n == 0) || (ld.n1 >= 0 && pd.n == 0);
     }
+    // what the code after the wait reads is loaded here (the compiler may
+    // otherwise move a load of read-only data down to its use)
+    asm volatile("" ::"f"(imp), "f"(d), "f"(sl), "f"(a));
     float si, fa;
-    if (!wait_values(on, slew + 4 * src + 2 * el + frf, at + 4 * src + 2 * el + frf, si, fa, ctl))
+    if (!wait_values(on, slew + 4 * R.x + 2 * el + frf, at + 4 * R.x + 2 * el + frf, si, fa, ctl))
       return false;
+    // sign(si) * sqrt(si^2 + impulse) at the sink (FlatRct::slew)
+    float at_sink = nanf(""), sink = nanf("");
+    if (s >= 0 && !none(si)) {
+      const float r = sqrtf(__fadd_rn(__fmul_rn(si, si), imp));
+      sink = si < 0.0f ? -r : r;
+    }
+    if (!none(fa) && !none(d)) at_sink = __fadd_rn(d, fa);
+    float arr = at_sink;  // what the arc brings to the pin
     if (thru) {
-      float so_u = nanf(""), at_u = nanf("");
-      if (t_s >= 0 && !none(si)) {
-        const float r = sqrtf(__fadd_rn(__fmul_rn(si, si), t_imp));
-        so_u = si < 0.0f ? -r : r;
-      }
-      if (!none(fa) && !none(t_d)) at_u = __fadd_rn(t_d, fa);
-      si = relax_fwd(el, t_psl, so_u);
-      fa = relax_fwd(el, t_pat, at_u);
+      si = sink;
+      fa = at_sink;
     }
-    if (kind == 0) {
-      // sign(si) * sqrt(si^2 + impulse) at the sink (FlatRct::slew)
-      if (s >= 0 && !none(si)) {
-        const float r = sqrtf(__fadd_rn(__fmul_rn(si, si), imp));
-        so = si < 0.0f ? -r : r;
-      }
-    } else if (none(si)) {
-      d = nanf("");
-    } else if (ps.n1 && pd.n1) {
-      so = prep_value(ps, si);
-      d = prep_value(pd, si);
+    if (!cell) {
+      so = sink;
+    } else if (slow || !(fabsf(si) < 3.402823466e+38f)) {
+      // rare: not one straight line for all of the warp's arcs
+      so = none(si) ? nanf("") : timing_value(lutd, ls, si, load);
+      d = none(si) ? nanf("") : timing_value(lutd, ld, si, load);
     } else {
-      so = timing_value(lutd, ls, si, load);
-      d = timing_value(lutd, ld, si, load);
+      int seg;
+      float t;
+      prep_segment(ps, si, seg, t);
+      so = prep_value(ps, seg, t);
+      if (!one_axis) prep_segment(pd, si, seg, t);
+      d = prep_value(pd, seg, t);
     }
-    if (!on) continue;
-    arc_delay[8 * (size_t)arc + (j & 7)] = d;
-    sl = relax_fwd(el, sl, so);
-    if (!none(fa) && !none(d)) a = relax_fwd(el, a, __fadd_rn(d, fa));
+    if (cell) arr = none(fa) || none(d) ? nanf("") : __fadd_rn(d, fa);
+    if (on) {
+      sl = relax_fwd(el, sl, so);
+      a = relax_fwd(el, a, arr);
+    }
+    if (j0 + 32 < nitems) {
+      if (on) arc_delay[8 * (size_t)arc + (j & 7)] = d;
+    } else {  // the last pass's delays are stored behind the pin's values
+      last_arc = on ? arc : -1;
+      last_d = d;
+    }
   }
-  __syncwarp();
   // lanes sharing (el, trf) differ in bits 1, 3 and 4
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
@@ -432,25 +503,26 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
     sl = relax_fwd(el, sl, __shfl_xor_sync(FULL, sl, m));
     a = relax_fwd(el, a, __shfl_xor_sync(FULL, a, m));
   }
-  // corner c's result sits in lane 4 * (c >> 1) + (c & 1); lane 0 stores
-  // the pin's slew and arrival time, which releases its readers, and marks
-  // its required time pending for the backward pass (the arc delays and
-  // test RATs are read only after the grid barrier)
-  float slc[4], atc[4];
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    slc[c] = canon(__shfl_sync(FULL, sl, 4 * (c >> 1) + (c & 1)));
-    atc[c] = canon(__shfl_sync(FULL, a, 4 * (c >> 1) + (c & 1)));
+  // corner c's result sits in lane 4 * (c >> 1) + (c & 1), which stores it:
+  // that releases the pin's readers.  Then the last arc delays, and the
+  // required time is marked pending for the backward pass (both, like the
+  // test RATs, are read only after the grid barrier)
+  sl = canon(sl);
+  a = canon(a);
+  if ((lane & ~5) == 0) {
+    st_relaxed(slew + 4 * v + c_out, sl);
+    st_relaxed(at + 4 * v + c_out, a);
+    rat[4 * v + c_out] = __uint_as_float(kPending);
   }
-  if (lane == 0) {
-    st_relaxed4(slew + 4 * v, slc[0], slc[1], slc[2], slc[3]);
-    st_relaxed4(at + 4 * v, atc[0], atc[1], atc[2], atc[3]);
-    const float p = __uint_as_float(kPending);
-    reinterpret_cast<float4*>(rat)[v] = make_float4(p, p, p, p);
-  }
+  if (last_arc >= 0) arc_delay[8 * (size_t)last_arc + (lane & 7)] = last_d;
+  after();
   // timing tests constrained at v (Test::_fprop_rat): lane j of a pass takes
   // test j/4 and output corner j%4
   const int t0 = __ldg(g.test_start + v), ntest = 4 * (__ldg(g.test_start + v + 1) - t0);
+  if (ntest == 0) return true;
+  float slc[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) slc[c] = __shfl_sync(FULL, sl, 4 * (c >> 1) + (c & 1));
   for (int j0 = 0; j0 < ntest; j0 += 32) {
     const int j = j0 + lane;
     const bool on = j < ntest;
@@ -478,6 +550,12 @@ __device__ bool fprop_warp(const G& G_, const LutSrc& lutd, int v, int lane, flo
     if (on) test_rat[4 * (size_t)test + (j & 3)] = val;
   }
   return true;
+}
+
+// MIN: arrival - required; MAX: required - arrival; empty if either is.
+__device__ __forceinline__ float slack_of(int c, float at, float rat) {
+  if (none(at) || none(rat)) return __uint_as_float(kEmpty);
+  return c < 2 ? __fsub_rn(at, rat) : __fsub_rn(rat, at);
 }
 
 // The net arcs among a driver's many fanouts, kNetArcs to a lane at a time,
@@ -552,7 +630,8 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
   const otg_prop_graph& g = G_.g;
   float r[4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) r[c] = lane == 0 ? __ldg(g.po_rat + 4 * v + c) : nanf("");
+  for (int c = 0; c < 4; ++c) r[c] = nanf("");
+  const float po = __ldg(g.po_rat + 4 * v + ((lane >> 1) & 3));  // of corner (bits 2, 1)
   const int t0 = __ldg(g.test_start + v), ntest = 4 * (__ldg(g.test_start + v + 1) - t0);
   const int o0 = __ldg(g.fanout_start + v), nout = __ldg(g.fanout_start + v + 1) - o0;
   int nitems = ntest + 8 * nout;
@@ -562,6 +641,9 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
     if (!bprop_net_arcs(g, o0, nout, lane, rat, arc_delay, r, &cells, ctl)) return false;
     if (!cells) nitems = ntest;
   }
+  // a single pass of arcs that only propagate: the candidates of corner
+  // (split, transition) sit in the lanes that agree in bits 2 and 1
+  const bool single = ntest == 0 && nitems <= 32 && !many;
   for (int j0 = 0; j0 < nitems; j0 += 32) {
     const int j = j0 + lane;
     int tc = 0;  // target corner
@@ -601,6 +683,7 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
         wa = __ldcg(at + 4 * w + 2 * wel + trf);
       }
     }
+    asm volatile("" ::"f"(dl), "f"(a), "f"(wa), "f"(po));
     float wr;
     if (!wait_value(mode != 0, rat + 4 * w + wc, wr, ctl)) return false;
     if (mode == 1) {
@@ -613,6 +696,18 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
       tc = 2 * MIN_ + frf;
       if (!none(a) && !none(wa) && !none(wr)) cand = __fsub_rn(a, __fsub_rn(wr, wa));
     }
+    if (single && !__any_sync(FULL, mode > 1)) {
+      const int sel = (lane >> 2) & 1, c = (lane >> 1) & 3;
+      float x = cand;
+#pragma unroll
+      for (int m : {1, 8, 16}) x = relax_bwd(sel, x, __shfl_xor_sync(FULL, x, m));
+      if (lane < 8 && (lane & 1) == 0) {
+        x = canon(relax_bwd(sel, x, po));
+        st_relaxed(rat + 4 * v + c, x);
+        slack[4 * v + c] = slack_of(c, __ldcg(at + 4 * v + c), x);
+      }
+      return true;
+    }
 #pragma unroll
     for (int c = 0; c < 4; ++c)
       if (c == tc) r[c] = relax_bwd(c >> 1, r[c], cand);
@@ -621,15 +716,15 @@ __device__ bool bprop_warp(const G& G_, int v, int lane, const float* at, float*
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int m = 1; m < 32; m <<= 1) r[c] = relax_bwd(c >> 1, r[c], __shfl_xor_sync(FULL, r[c], m));
+#pragma unroll
+  for (int c = 0; c < 4; ++c) r[c] = relax_bwd(c >> 1, r[c], __shfl_sync(FULL, po, 2 * c));
   if (lane == 0) {
     st_relaxed4(rat + 4 * v, canon(r[0]), canon(r[1]), canon(r[2]), canon(r[3]));
     const float4 a4 = __ldcg(reinterpret_cast<const float4*>(at) + v);
     const float a[4] = {a4.x, a4.y, a4.z, a4.w};
     float sk[4];
 #pragma unroll
-    for (int c = 0; c < 4; ++c)
-      sk[c] = (none(a[c]) || none(r[c])) ? __uint_as_float(kEmpty)
-              : (c < 2 ? __fsub_rn(a[c], r[c]) : __fsub_rn(r[c], a[c]));
+    for (int c = 0; c < 4; ++c) sk[c] = slack_of(c, a[c], r[c]);
     reinterpret_cast<float4*>(slack)[v] = make_float4(sk[0], sk[1], sk[2], sk[3]);
   }
   return true;
@@ -646,8 +741,13 @@ __device__ __forceinline__ bool pin_on(const int32_t* pin_group, const uint8_t* 
 // the list's length.)
 __global__ void prop_init_kernel(float4* at, float4* slew, int num_pins, GridCtl* ctl,
                                  const int32_t* pin_group, const uint8_t* group_active,
-                                 const int32_t* items, int all_pins) {
+                                 const int32_t* items, int all_pins, G G_, int4* rec) {
   const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool all = !items && !pin_group;
+  if (all)
+    for (int f = i0, n = min(__ldg(G_.g.fanin_start + all_pins), G_.g.num_arcs); f < n;
+         f += gridDim.x * blockDim.x)
+      rec[f] = fanin_rec(G_, __ldg(G_.g.fanin + f));
   if (i0 == 0 && !items) *ctl = GridCtl{0u, 0u, 0, 0};
   const float p = __uint_as_float(kPending);
   for (int k = i0; k < num_pins; k += gridDim.x * blockDim.x) {
@@ -659,33 +759,70 @@ __global__ void prop_init_kernel(float4* at, float4* slew, int num_pins, GridCtl
     if (!pin_on(pin_group, group_active, i)) continue;
     at[i] = make_float4(p, p, p, p);
     slew[i] = make_float4(p, p, p, p);
+    if (!all) {
+      const int f1 = min(__ldg(G_.g.fanin_start + i + 1), G_.g.num_arcs);
+      for (int f = __ldg(G_.g.fanin_start + i); f < f1; ++f)
+        rec[f] = fanin_rec(G_, __ldg(G_.g.fanin + f));
+    }
   }
 }
 
 // The whole propagation in one cooperative launch; warp w of W takes items
-// w, w + W, ... of each pass.
-__global__ void __launch_bounds__(256) prop_kernel(G G_, const int* order, const int* fwd_order,
-                                                   int num_pins,
-                                                   float* at, float* slew, float* rat,
-                                                   float* slack, float* arc_delay,
-                                                   float* test_rat, GridCtl* ctl, int lut_smem,
-                                                   const int32_t* pin_group,
-                                                   const uint8_t* group_active) {
+// w, w + W, ... of each pass.  kCtas CTAs per SM: where a warp has many
+// pins, more warps count (four CTAs, 64 registers: 240k gates 1.34 ms
+// against 1.86 with two), where it has few, the chain of waits does (two,
+// 103 registers, no spills on it: 2k gates 194 us against 216).
+template <int kCtas>
+__global__ void __launch_bounds__(kPropT, kCtas)
+    prop_kernel(G G_, const int* order, const int* fwd_order, int num_pins, float* at, float* slew,
+                float* rat, float* slack, float* arc_delay, float* test_rat, GridCtl* ctl,
+                int lut_smem, const int32_t* pin_group, const uint8_t* group_active,
+                const int4* rec) {
   // the library's tables, staged on chip when the caller gave their size
   // and they fit (lut_smem floats)
   extern __shared__ float s_lut[];
   for (int i = threadIdx.x; i < lut_smem; i += blockDim.x) s_lut[i] = __ldg(G_.g.lut_data + i);
   __syncthreads();
   const LutSrc lutd{s_lut, lut_smem, G_.g.lut_data};
+  const int prep0 = lut_smem;  // the prepared tables follow
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int W = (gridDim.x * blockDim.x) >> 5;
   bool ok = true;
-  for (int j = warp; ok && j < num_pins; j += W) {
-    const int v = fwd_order ? __ldg(fwd_order + j) : __ldg(order + num_pins - 1 - j);
-    if ((unsigned)v >= (unsigned)G_.g.num_pins) continue;  // a bad item (reported by the fill)
-    if (!pin_on(pin_group, group_active, v)) continue;
-    ok = fprop_warp(G_, lutd, v, lane, at, slew, rat, arc_delay, test_rat, ctl);
+  // the pin of item j (-1: none, a bad item (reported by the fill), or one
+  // whose group is off)
+  auto pin = [&](const int* list, bool down, int j) {
+    if (j >= num_pins) return -1;
+    const int v = __ldg(list + (down ? num_pins - 1 - j : j));
+    return (unsigned)v < (unsigned)G_.g.num_pins && pin_on(pin_group, group_active, v) ? v : -1;
+  };
+  auto range = [&](const int* start, Visit& x) {
+    x.lo = x.v >= 0 ? __ldg(start + x.v) : 0;
+    x.hi = x.v >= 0 ? __ldg(start + x.v + 1) : 0;
+  };
+  {
+    const int* list = fwd_order ? fwd_order : order;
+    const bool down = !fwd_order;
+    auto first = [&](Visit& x) {
+      const int f = x.lo + (lane >> 3);
+      x.rec = f < x.hi ? __ldg(rec + f) : kNoRec;
+    };
+    Visit me, next;
+    me.v = pin(list, down, warp);
+    range(G_.g.fanin_start, me);
+    first(me);
+    next.v = pin(list, down, warp + W);
+    for (int j = warp; ok && j < num_pins; j += W) {
+      const int v2 = pin(list, down, j + 2 * W);
+      range(G_.g.fanin_start, next);
+      if (me.v >= 0)
+        ok = fprop_warp(G_, rec, lutd, prep0, me, lane, at, slew, rat, arc_delay, test_rat, ctl,
+                        [&] { first(next); });
+      else
+        first(next);
+      me = next;
+      next.v = v2;
+    }
   }
   // the barrier also lets every CTA leave together when a wait gave up
   if (!grid_barrier(ctl) || !ok) return;
@@ -705,10 +842,20 @@ size_t align256p(size_t x) { return (x + 255) & ~(size_t)255; }
 // takes about 33 KB).
 constexpr int kLutSmemFloats = 10240;
 
+// Dynamic shared memory of the kernel with lut_smem floats of staged tables.
+size_t prop_smem(int lut_smem) {
+  return 4 * ((size_t)lut_smem + kPrepFloats * (lut_smem ? 1 : 2));
+}
+
+// Up to this many pins per warp at two CTAs per SM, those are launched
+// (2k gates have 2, a 6k-gate block 8: 666 us against 718; 60k gates 69:
+// 657 against 645).
+constexpr int kFewPins = 32;
+
 struct PropDev {
   int sms = 0;
-  int occ[2] = {0, 0};  // CTAs per SM without / with the staged tables
   bool init = false;
+  std::atomic<long long> occ[2];  // per variant, of its last launch: (lut_smem + 1) << 32 | CTAs per SM
 };
 PropDev g_pdev[64];
 
@@ -720,7 +867,8 @@ extern "C" {
 otg_status otg_prop_workspace_size(int32_t num_pins, int32_t num_arcs, int32_t num_tests,
                                    size_t* bytes) {
   if (!bytes || num_pins < 0 || num_arcs < 0 || num_tests < 0) return OTG_ERR_INVALID;
-  *bytes = 256 + otg::align256p(32 * (size_t)num_arcs) + otg::align256p(16 * (size_t)num_tests);
+  *bytes = 256 + otg::align256p(32 * (size_t)num_arcs) + otg::align256p(16 * (size_t)num_tests) +
+           otg::align256p(sizeof(int4) * (size_t)num_arcs);
   return OTG_OK;
 }
 
@@ -755,8 +903,11 @@ static otg_status propagate_impl(const otg_prop_graph* g, const otg_prop_rc* rc,
   // with items, the fill may record a bad item, so the control block is
   // cleared before it (without items the fill clears it itself)
   if (items && cudaMemsetAsync(ctl, 0, sizeof(otg::GridCtl), st) != cudaSuccess) return OTG_ERR_CUDA;
-  otg::prop_init_kernel<<<std::max(1, std::min(1184, (P + 255) / 256)), 256, 0, st>>>(
-      (float4*)at, (float4*)slew, P, ctl, pin_group, group_active, items, g->num_pins);
+  int4* rec = (int4*)((char*)test_rat + otg::align256p(16 * (size_t)g->num_tests));
+  otg::G G_{*g, *rc};
+  const int work = items || pin_group ? P : std::max(P, (int)g->num_arcs);
+  otg::prop_init_kernel<<<std::max(1, std::min(1184, (work + 255) / 256)), 256, 0, st>>>(
+      (float4*)at, (float4*)slew, P, ctl, pin_group, group_active, items, g->num_pins, G_, rec);
   otg::count_launch();
   if (cudaGetLastError() != cudaSuccess) return OTG_ERR_CUDA;
   if (P == 0) return OTG_OK;
@@ -765,26 +916,33 @@ static otg_status propagate_impl(const otg_prop_graph* g, const otg_prop_rc* rc,
   otg::PropDev& d = otg::g_pdev[dev & 63];
   if (!d.init) {
     cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaFuncSetAttribute(otg::prop_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         4 * otg::kLutSmemFloats);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ[0], otg::prop_kernel, 256, 0);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&d.occ[1], otg::prop_kernel, 256,
-                                                  4 * otg::kLutSmemFloats);
+    for (auto k : {otg::prop_kernel<2>, otg::prop_kernel<4>})
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)otg::prop_smem(otg::kLutSmemFloats));
     d.init = true;
   }
   int lut_smem = g->num_lut_data > 0 && g->num_lut_data <= otg::kLutSmemFloats ? g->num_lut_data : 0;
-  const int occ = lut_smem ? d.occ[1] : d.occ[0];
+  const size_t smem = otg::prop_smem(lut_smem);
+  const bool few = P <= otg::kFewPins * 2 * d.sms * (otg::kPropT / 32);
+  auto kern = few ? otg::prop_kernel<2> : otg::prop_kernel<4>;
+  long long known = d.occ[few].load(std::memory_order_relaxed);
+  if ((known >> 32) != lut_smem + 1) {
+    int o = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, otg::kPropT, smem);
+    known = ((long long)(lut_smem + 1) << 32) | std::min(o, few ? 2 : 4);
+    d.occ[few].store(known, std::memory_order_relaxed);
+  }
+  const int occ = (int)(known & 0xFFFFFFFFll);
   // every CTA resident (the schedule and the barrier rely on it), no more
   // warps than pins
   const int grid = std::max(1, std::min(d.sms * std::max(occ, 1), (P + 7) / 8));
-  otg::G G_{*g, *rc};
   int num_pins = P;
   void* args[] = {&G_,       (void*)&order, (void*)&fwd_order, &num_pins,
                   &at,       &slew,         &rat,              &slack,
                   &arc_delay, &test_rat,    &ctl,              &lut_smem,
-                  (void*)&pin_group, (void*)&group_active};
+                  (void*)&pin_group, (void*)&group_active, &rec};
   const cudaError_t e = cudaLaunchCooperativeKernel(
-      (const void*)otg::prop_kernel, dim3(grid), dim3(256), args, 4 * (size_t)lut_smem, st);
+      (const void*)kern, dim3(grid), dim3(otg::kPropT), args, smem, st);
   otg::count_launch();
   if (e != cudaSuccess) {
     cudaGetLastError();
