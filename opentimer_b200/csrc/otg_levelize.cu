@@ -2,37 +2,41 @@
 //
 // Replaces toposort_advance + toposort_compute_cuda (ot/cuda/toposort.cu:4-72)
 // which launch one kernel per level and copy the frontier size back to the
-// host after each one.  Here every level runs inside ONE cooperative launch:
+// host after each one.  Here:
+//   pack    every pin's fanins as one 16-byte record (the whole GPU);
+//   levels  one launch for all levels: level 0 is the caller's seed (pins
+//           without candidate fanout); expanding a level decrements the
+//           fanout counter of each fanin of its pins, and a pin whose
+//           counter reaches zero belongs to the next level;
+//   sort    the pins by (level, pin index) -- every level after the seed
+//           comes out in ascending pin order, deterministically -- and the
+//           levels' ends.
+// A level is a chain of round trips, so the chain is kept short.  The step
+// that decrements a pin's counter loads its record too: a pin that becomes
+// ready enters the next level's list, in its CTA's shared memory, with its
+// fanins, and that level starts its decrements from there, four lanes an
+// entry: no fanin range to look up, no scan and no search to spread edges
+// over threads, nothing read back.  Order and level ends are not on the
+// chain at all.  A barrier, the counter's atomic and the list append are
+// what is left.
 //
-//   level 0      = the caller's seed (pins without candidate fanout)
-//   expand(k)    every pin of level k decrements the fanout counter of each
-//                of its fanins, edge-parallel: a block scan over the pins'
-//                fanin counts hands one edge to each thread, so all of a
-//                chunk's decrements are in flight at once (warp-aggregated
-//                atomics: lanes that hit the same pin combine into one
-//                atomicSub); the pin whose counter reaches zero sets its bit
-//                in the "ready" bitmap
-//   compact(k+1) the ready bitmap is split into per-CTA word ranges of C
-//                words.  The expansion that sets a pin's bit also counts it
-//                for its range, so after ONE grid barrier every CTA knows its
-//                offset (the counts of the ranges before it), writes its pins
-//                in ascending index order there -- every level after the seed
-//                comes out sorted by pin index, deterministically -- and
-//                expands them into the other bitmap.  The range counts rotate
-//                through three buffers: read in level k, filled for k+1,
-//                cleared for k+2.
-//
-// One grid barrier per level.  The barrier is a sense-counting barrier on
-// global memory whose waits are bounded by %globaltimer: a wait that runs
-// past the limit raises an abort flag that every other wait also watches,
-// so the kernel always returns and the host sees OTG_ERR_TIMEOUT.
-//
-// Graphs of up to about a million pins run instead in ONE thread-block
-// cluster (levelize_cluster_kernel below):
-// the same rule and the same outputs, with the ready bitmaps and counts in
-// distributed shared memory, the hardware cluster barrier between levels,
-// and the next level's fanin ranges gathered while the counters are
-// decremented.
+// Two forms of the levels kernel, with the same outputs:
+//   cluster  graphs of up to 650k pins run in ONE thread-block cluster: the
+//            counters lie in the CTAs' shared memory, and a level ends at
+//            the hardware cluster barrier;
+//   grid     larger graphs run on every SM, counters in global memory, one
+//            grid barrier per level.  It is a sense-counting barrier whose
+//            waits are bounded by %globaltimer: a wait that runs past the
+//            limit raises an abort flag that every other wait also watches,
+//            so the kernel always returns and the host sees OTG_ERR_TIMEOUT.
+// Before, a level's pins were found in ready bitmaps, written out in order,
+// and their fanins looked up, scanned and searched by thread, all on the
+// chain: 2.53 ms on 5M pins / 200 levels (grid; now 1.47), 1.30 ms on a
+// 60k-gate design's 163k pins / 374 levels (cluster; now 0.55).  What bounds
+// it now is the chain still: per level one barrier, one counter round trip
+// and the appends, 1.4 us in the cluster and 2.6 us on the grid where a
+// level has few pins.  32-byte records of eight fanins were 15-20% slower
+// (their copies into the lists).
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -47,639 +51,567 @@
 namespace otg {
 namespace {
 
-constexpr unsigned FULL = 0xffffffffu;
-constexpr int LT = 512;                              // threads per CTA
-using LvCtl = GridCtl;
-
-// One fanin edge per lane (target v, ok = a valid pin): decrement v's
-// fanout counter; the pin whose counter reaches zero sets its bit in `bm`
-// and counts for its range.  Lanes of a warp that target the same pin
-// combine into one atomicSub.  Every lane of the warp must call it.  A
-// seed pin's counter starts at INT_MAX, so a seed is never emitted twice,
-// even if the caller's out_deg disagrees with the fanin lists, and no
-// other read is needed on this chain.
-__device__ __forceinline__ void decrement(int v, bool ok, int* cnt, unsigned* bm, int* rcount,
-                                          int C) {
-  const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(FULL, ok ? v : -2 - lane);
-  if (ok && (__ffs(peers) - 1 == lane)) {
-    const int k = __popc(peers);
-    const int old = atomicSub(&cnt[v], k);
-    if (old > 0 && old - k <= 0) {
-      atomicOr(&bm[v >> 5], 1u << (v & 31));
-      atomicAdd(&rcount[(v >> 5) / C], 1);
-    }
-  }
-}
-
-// Decrement the fanout counters of u's fanins, one edge per lane per step
-// (the seed level).
-__device__ __forceinline__ void expand_pin(int u, bool active, const int* fanin_start,
-                                           const int* fanin, int* cnt, unsigned* bm, int n,
-                                           int* rcount, int C) {
-  int e = active ? fanin_start[u] : 0;
-  const int e1 = active ? fanin_start[u + 1] : 0;
-  while (__any_sync(FULL, e < e1)) {
-    const bool has = e < e1;
-    const int v = has ? fanin[e] : -1;
-    decrement(v, has && (unsigned)v < (unsigned)n, cnt, bm, rcount, C);
-    e += has ? 1 : 0;
-  }
-}
-
-__global__ void __launch_bounds__(LT) levelize_kernel(int n, const int* fanin_start,
-                                                      const int* fanin, const int* out_deg,
-                                                      const int* frontier0, int first_size,
-                                                      int* order, int* level, int* level_ends,
-                                                      int* counts, LvCtl* ctl, int* cnt,
-                                                      unsigned* bm0, unsigned* bm1, int* blk) {
-  // blk: three rotating [G] buffers of per-range ready counts
-  __shared__ int wsum[LT / 32];
-  __shared__ int red_t[LT / 32], red_b[LT / 32];
-  __shared__ int s_estart[LT], s_e0[LT];
-  __shared__ int s_total, s_off;
-  const int G = gridDim.x, b = blockIdx.x, tid = threadIdx.x;
-  const int gtid = b * LT + tid, gstride = G * LT;
-  const int nw = (n + 31) >> 5;
-  const int lane = tid & 31, w = tid >> 5;
-
-  for (int v = gtid; v < n; v += gstride) {
-    cnt[v] = out_deg[v];
-    level[v] = -1;
-  }
-  for (int i = gtid; i < nw; i += gstride) bm0[i] = bm1[i] = 0u;
-  for (int i = gtid; i < 3 * G; i += gstride) blk[i] = 0;
-  const int C = max(1, (nw + G - 1) / G);  // bitmap words per CTA range
-  if (!grid_barrier(ctl)) return;
-  for (int k = gtid; k < first_size; k += gstride) {
-    const int v = frontier0[k];
-    order[k] = v;
-    if ((unsigned)v < (unsigned)n) {
-      level[v] = 0;
-      cnt[v] = INT_MAX;  // after the counters' fill (grid barrier above)
-    } else {
-      atomicCAS(&ctl->status, 0, (int)OTG_ERR_INVALID);
-    }
-  }
-  if (gtid == 0) {
-    level_ends[0] = 0;
-    if (first_size > 0) level_ends[1] = first_size;
-  }
-  if (first_size == 0) {
-    if (gtid == 0) { counts[0] = 0; counts[1] = 0; }
-    return;
-  }
-  if (!grid_barrier(ctl)) return;
-  // expand the seed
-  for (int k0 = b * LT; k0 < first_size; k0 += gstride) {
-    const int k = k0 + tid;
-    const bool act = k < first_size && (unsigned)order[k] < (unsigned)n;
-    expand_pin(act ? order[k] : 0, act, fanin_start, fanin, cnt, bm0, n, blk + G, C);
-  }
-  unsigned* cur = bm0;
-  unsigned* nxt = bm1;
-  int emitted = first_size;
-  int L = 1;
-  const int w0 = min(nw, b * C), w1 = min(nw, (b + 1) * C);
-  while (true) {
-    if (!grid_barrier(ctl)) return;
-    int* rc_now = blk + (L % 3) * G;         // counts of this level's ranges
-    int* rc_next = blk + ((L + 1) % 3) * G;  // filled by this level's expansion
-    if (tid == 0) blk[((L + 2) % 3) * G + b] = 0;  // read a level ago, filled next level
-    // the first tile's bitmap words load while the counts are summed
-    unsigned word0[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      word0[j] = w0 + 2 * tid + j < w1 ? __ldcg(cur + w0 + 2 * tid + j) : 0u;
-    // offset of this CTA and level total: every thread reads at most a few
-    // counts (independent loads), then a block reduction
-    {
-      int before = 0, total = 0;
-      for (int i = tid; i < G; i += LT) {
-        const int x = __ldcg(rc_now + i);
-        total += x;
-        if (i < b) before += x;
-      }
-      for (int d = 16; d >= 1; d >>= 1) {
-        total += __shfl_xor_sync(FULL, total, d);
-        before += __shfl_xor_sync(FULL, before, d);
-      }
-      if (lane == 0) { red_t[w] = total; red_b[w] = before; }
-      __syncthreads();
-      if (tid == 0) {
-        int t = 0, o = 0;
-        for (int k = 0; k < LT / 32; ++k) { t += red_t[k]; o += red_b[k]; }
-        s_total = t;
-        s_off = o;
-      }
-      __syncthreads();
-    }
-    const int total = s_total;
-    if (total == 0) break;
-    int run = emitted + s_off;
-    // write own pins in ascending order, tile by tile (two bitmap words per
-    // thread), and expand them
-    for (int t0 = w0; t0 < w1; t0 += 2 * LT) {
-      const int i = t0 + 2 * tid;
-      unsigned wd[2];
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-        wd[j] = t0 == w0 ? word0[j] : (i + j < w1 ? __ldcg(cur + i + j) : 0u);
-      const int pc = __popc(wd[0]) + __popc(wd[1]);
-      // block exclusive scan of pc
-      int x = pc;
-      for (int d = 1; d < 32; d <<= 1) {
-        const int y = __shfl_up_sync(FULL, x, d);
-        if (lane >= d) x += y;
-      }
-      if (lane == 31) wsum[w] = x;
-      __syncthreads();
-      int wb = 0, tt = 0;
-      for (int u = 0; u < LT / 32; ++u) {
-        if (u < w) wb += wsum[u];
-        tt += wsum[u];
-      }
-      __syncthreads();
-      int pos = run + wb + x - pc;
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        unsigned bits = wd[j];
-        while (bits) {
-          const int bit = __ffs(bits) - 1;
-          bits &= bits - 1;
-          const int v = ((i + j) << 5) + bit;
-          if (pos < n) {
-            order[pos] = v;
-          } else {
-            atomicCAS(&ctl->status, 0, (int)OTG_ERR_INVALID);  // duplicate seeds
-          }
-          ++pos;
-          level[v] = L;
-        }
-        if (i + j < w1) cur[i + j] = 0u;  // ready for reuse two levels on
-      }
-      __syncthreads();  // the tile's slice of `order` is visible to the CTA
-      // expand the tile's pins edge-parallel: LT pins at a time, their fanin
-      // edges spread one per thread, so every decrement of a chunk is in
-      // flight at once instead of one edge after another per pin
-      const int tn = min(tt, n - run);
-      for (int c0 = 0; c0 < tn; c0 += LT) {
-        const int k = c0 + tid;
-        int e0 = 0, deg = 0;
-        if (k < tn) {
-          const int u = order[run + k];
-          if ((unsigned)u < (unsigned)n) {
-            e0 = fanin_start[u];
-            deg = fanin_start[u + 1] - e0;
-          }
-        }
-        // block exclusive scan of the degrees
-        int y = deg;
-        for (int d = 1; d < 32; d <<= 1) {
-          const int z = __shfl_up_sync(FULL, y, d);
-          if (lane >= d) y += z;
-        }
-        if (lane == 31) wsum[w] = y;
-        __syncthreads();
-        int eb = 0, etot = 0;
-        for (int u = 0; u < LT / 32; ++u) {
-          if (u < w) eb += wsum[u];
-          etot += wsum[u];
-        }
-        s_estart[tid] = eb + y - deg;
-        s_e0[tid] = e0;
-        __syncthreads();
-        const int np = min(LT, tn - c0);
-        for (int q0 = 0; q0 < etot; q0 += LT) {
-          const int q = q0 + tid;
-          int v = -1;
-          if (q < etot) {
-            // the pin owning edge q: the last one whose start is <= q
-            int lo = 0, hi = np - 1;
-            while (lo < hi) {
-              const int mid = (lo + hi + 1) >> 1;
-              if (s_estart[mid] <= q) lo = mid; else hi = mid - 1;
-            }
-            v = fanin[s_e0[lo] + (q - s_estart[lo])];
-          }
-          decrement(v, (unsigned)v < (unsigned)n, cnt, nxt, rc_next, C);
-        }
-        __syncthreads();  // s_estart / s_e0 / wsum are reused
-      }
-      run += tt;
-    }
-    emitted += total;
-    if (emitted > n) {  // only reachable with duplicate seeds; stop cleanly
-      if (gtid == 0) atomicCAS(&ctl->status, 0, (int)OTG_ERR_INVALID);
-      emitted = n;
-      break;
-    }
-    if (gtid == 0) level_ends[L + 1] = emitted;
-    ++L;
-    unsigned* t = cur;
-    cur = nxt;
-    nxt = t;
-  }
-  if (gtid == 0) {
-    counts[0] = L;
-    counts[1] = emitted;
-  }
-}
-
-// ---- the cluster path --------------------------------------------------
-//
-// Graphs whose two ready bitmaps fit in the shared memory of one thread-
-// block cluster (up to 16 CTAs, 8 or fewer where the device cannot place
-// 16) run the same frontier rule inside one cluster: CTA r owns the bitmap
-// words [r*C, (r+1)*C) of both levels in its own shared memory, and a pin
-// whose fanout counter reaches zero sets its bit and bumps its owner's
-// count through distributed shared memory.  A level ends at the hardware
-// cluster barrier (barrier.cluster, release/acquire) instead of the global
-// barrier, and the counts and bitmaps never leave the SMs.  Where the
-// ranges' fanout counters fit beside them (32 ints per bitmap word), the
-// counters live in their owner's shared memory too, and a level costs the
-// dependent global loads of its expansion (the fanin entry; the fanin
-// range, loaded speculatively beside the decrement) plus on-chip work.
-// The emission rule is the one
-// above (seed order, then ascending pin index per level, CTA ranges in rank
-// order), so both paths give identical outputs.
-//
-// No wait in this path polls memory: the cluster barrier is hardware, and
-// every CTA takes the same number of barriers (the loop ends on the level
-// total, which every CTA computes from the same counts).
-
-// CTA widths of the cluster path: a level of a narrow graph has a few pins
-// per CTA, and every warp of the CTA takes part in each of its scans and
-// barriers, so narrow graphs run narrow CTAs.
-constexpr int kCtMax = 1024;
-
-// Optional per-segment cycle accounting of the level loop (build with
-// -DOTG_PHASE_TIMING): thread 0 of CTA 0 sums the clock64() deltas of each
-// segment and stores them after the counts, in counts[2..9] (the caller
-// then passes a counts array of 10).
-#ifdef OTG_PHASE_TIMING
-#define LV_PHASE_BEGIN() long long _ph_t = clock64(), _ph[8] = {0, 0, 0, 0, 0, 0, 0, 0}
-#define LV_PHASE(k)                        \
-  do {                                     \
-    if (gtid == 0) {                       \
-      const long long _t = clock64();      \
-      _ph[k] += _t - _ph_t;                \
-      _ph_t = _t;                          \
-    }                                      \
-  } while (0)
-#define LV_PHASE_END(c)                                                   \
-  do {                                                                    \
-    if (gtid == 0)                                                        \
-      for (int _k = 0; _k < 8; ++_k) (c)[2 + _k] = (int)(_ph[_k] >> 10); \
-  } while (0)
-#else
-#define LV_PHASE_BEGIN() \
-  do {                   \
-  } while (0)
-#define LV_PHASE(k) \
-  do {              \
-  } while (0)
-#define LV_PHASE_END(c) \
-  do {                  \
-  } while (0)
-#endif
-
 namespace cg = cooperative_groups;
+constexpr unsigned FULL = 0xffffffffu;
 
-// Where a pin that becomes ready goes: its owner's bitmap word and count
-// (distributed shared memory), and the list of fanin ranges that one CTA,
-// chosen by a hash of the pin, expands next level.  (Hashing keeps the
-// lists even: a CTA that readied a whole level -- a buffer tree readies
-// its levels from one place -- would otherwise expand the next one alone.)
-struct ClNext {
-  unsigned* bm;  // next level's bitmap (this CTA's address; mapped to the owner)
-  int* scnt;     // the fanin counters of the CTA's range (mapped to the owner), or null:
-                 // the counters are the global cnt[]
-  int cshift;    // log2 of the words per CTA range: the owner of word w is w >> cshift
-  int sshift;    // log2 of the cluster size
-  int* rc;       // next level's per-owner counts [16] (every CTA keeps a copy)
-  int2* lst;     // next level's list of (fanin start, fanin count) (mapped to the target)
-  int* lcnt;     // its length (likewise)
-  int* ovf;      // next level's overflow flag (set in every CTA)
-  int cap;       // list capacity
+// A pin's fanins: up to four (-1: none), or {first index in fanin[], their
+// number, 0, kWide}.  In the lists a wide record names at most kWideMax
+// fanins, a quad of lanes' worth, unless it has more than kWideLong.
+constexpr int kWide = -2, kWideMax = 4, kWideLong = 64;
+
+struct LvCtl {
+  GridCtl grid;
+  int levels;    // found by the levels kernel
+  int tot[4];    // ready pins' list entries of a level, by level (grid form)
+  int spill[4];  // pins in the level's spill list
 };
 
-// One fanin edge per lane (as decrement above).  The leader lane of each
-// distinct pin v also loads v's fanin range, in flight with the decrement,
-// so a pin that becomes ready is expanded next level without another
-// global round trip; a full list raises the next level's overflow flag in
-// every CTA, and that level then expands from the bitmaps instead.  The
-// counter lives in the owner's shared memory where the ranges fit there
-// (a distributed-shared-memory atomic instead of an L2 round trip on every
-// level's critical path).  The warp's pins that became ready add to the
-// per-owner counts of every CTA once per owner.
-__device__ __forceinline__ void decrement_cl(int v, bool ok, const int* fanin_start, int* cnt,
-                                             const ClNext& nx, const cg::cluster_group& cl) {
-  const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(FULL, ok ? v : -2 - lane);
-  bool ready = false;
-  int owner = 0;
-  if (ok && (__ffs(peers) - 1 == lane)) {
-    const int k = __popc(peers);
-    const int s0 = __ldg(fanin_start + v), s1 = __ldg(fanin_start + v + 1);
-    const int w = v >> 5;
-    owner = w >> nx.cshift;
-    int* c = nx.scnt ? cl.map_shared_rank(nx.scnt + (v - (owner << (nx.cshift + 5))), owner)
-                     : cnt + v;
-    const int old = atomicSub(c, k);
-    if (old > 0 && old - k <= 0) {
-      ready = true;
-      atomicOr(cl.map_shared_rank(nx.bm, owner) + (w - (owner << nx.cshift)), 1u << (v & 31));
-      const int t = nx.sshift ? (int)(((unsigned)v * 0x9E3779B1u) >> (32 - nx.sshift)) : 0;
-      const int slot = atomicAdd(cl.map_shared_rank(nx.lcnt, t), 1);
-      if (slot < nx.cap) {
-        *cl.map_shared_rank(nx.lst + slot, t) = make_int2(s0, s1 - s0);
-      } else {
-        for (int i = 0; i < (int)cl.num_blocks(); ++i) *cl.map_shared_rank(nx.ovf, i) = 1;
-      }
+struct LvArgs {
+  int n;
+  const int* fanin_start;
+  const int* fanin;
+  const int* out_deg;
+  const int* frontier0;
+  int first_size;
+  int* order;
+  int* level;
+  int* level_ends;
+  int* counts;
+  LvCtl* ctl;
+  int* cnt;      // fanout counters (unless they lie on chip)
+  int4* packed;  // records by pin; behind the levels, the sort's scratch
+  int* spill;    // two lists of n pins, by level parity: what no CTA's list held
+};
+
+__global__ void levelize_pack(LvArgs a, bool counters) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i0 == 0) *a.ctl = LvCtl{};
+  for (int v = i0; v < a.n; v += gridDim.x * blockDim.x) {
+    const int e0 = a.fanin_start[v], deg = a.fanin_start[v + 1] - e0;
+    int f[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int u = k < deg && deg <= 4 ? a.fanin[e0 + k] : -1;
+      f[k] = (unsigned)u < (unsigned)a.n ? u : -1;
     }
-  }
-  const unsigned grp = __match_any_sync(FULL, ready ? owner : -1 - lane);
-  if (ready && (__ffs(grp) - 1 == lane)) {
-    const int k = __popc(grp), S = (int)cl.num_blocks();
-    for (int i = 0; i < S; ++i) atomicAdd(cl.map_shared_rank(nx.rc + owner, i), k);
+    a.packed[v] = deg > 4 ? make_int4(e0, deg, 0, kWide) : make_int4(f[0], f[1], f[2], f[3]);
+    a.level[v] = -1;
+    if (counters) a.cnt[v] = a.out_deg[v];
   }
 }
+
+// ---- the lists.  A CTA holds two (by level parity) of `cap` records and
+// their pins (-1 in a record that continues the one before).
+struct LvLists {
+  int4* rec0;  // the even levels' records, then the odd ones'
+  int* pin0;   // likewise their pins
+  int cap;
+  __device__ int4* rec(int L) const { return rec0 + (L & 1) * cap; }
+  __device__ int* pin(int L) const { return pin0 + (L & 1) * cap; }
+};
+
+// Puts pin v's record into list entries [at, at + recs) of a list; entries
+// past the capacity are left out.  False if some were.
+__device__ __forceinline__ bool put_records(int4* rec, int* pin, int cap, int at, int recs, int v,
+                                            int4 pk) {
+  const bool fits = at + recs <= cap;
+  for (int k = 0; k < recs; ++k) {
+    if (at + k >= cap) break;
+    int4 x = pk;
+    if (recs > 1)
+      x = make_int4(pk.x + kWideMax * k, min(kWideMax, pk.y - kWideMax * k), 0, kWide);
+    rec[at + k] = fits ? x : make_int4(-1, -1, -1, -1);
+    pin[at + k] = fits && k == 0 ? v : -1;
+  }
+  return fits;
+}
+
+__device__ __forceinline__ void spill_pin(const LvArgs& a, int v, int L) {
+  a.spill[(size_t)(L & 1) * a.n + atomicAdd(&a.ctl->spill[L & 3], 1)] = v;
+}
+
+// One fanin edge per lane (target v, or none): decrement v's fanout counter;
+// a pin whose counter reaches zero is of level L.  Every lane of the warp
+// must call it.  A seed pin's counter starts at INT_MAX, so a seed is never
+// emitted twice.  (Lanes with the same target do not combine: finding them
+// takes match_any 380 cycles when the targets differ, 1100 with every warp
+// at it, against 440 for the counter's round trip.)
+// The group gives the counter's place, this CTA's list length for L, how
+// long that may grow, and takes what it does not hold (hand_on).
+template <class Gp>
+__device__ __forceinline__ void decrement(const Gp& g, const LvArgs& a, const LvLists& ls, int v,
+                                          int L) {
+  const int lane = threadIdx.x & 31;
+  bool ready = false;
+  int4 pk = make_int4(-1, -1, -1, -1);
+  if ((unsigned)v < (unsigned)a.n) {
+    pk = __ldcg(a.packed + v);
+    ready = atomicSub(g.counter(v), 1) == 1;
+  }
+  const unsigned set = __ballot_sync(FULL, ready);
+  if (set == 0u) return;
+  const int recs =
+      !ready ? 0
+             : (pk.w == kWide && pk.y <= kWideLong ? (pk.y + kWideMax - 1) / kWideMax : 1);
+  int at = __popc(set & ((1u << lane) - 1u)), total = __popc(set);
+  if (__any_sync(FULL, recs > 1)) {
+    int upto = recs;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(FULL, upto, d);
+      if (lane >= d) upto += y;
+    }
+    at = upto - recs;
+    total = __shfl_sync(FULL, upto, 31);
+  }
+  int* len = g.length(L);
+  int base = -1;
+  if (lane == 0 && *(volatile int*)len < g.most()) base = atomicAdd(len, total);
+  base = __shfl_sync(FULL, base, 0);
+  if (ready) {
+    if (base < 0) g.hand_on(v, pk, recs, L);
+    else if (!put_records(ls.rec(L), ls.pin(L), ls.cap, base + at, recs, v, pk))
+      g.spill(v, L);
+  }
+}
+
+// Decrements for the records get(0), get(1), ..., get(m - 1), a quad of
+// lanes each (get(k, f): word f of record k), by `threads` threads of which
+// this is number `at`; the pins made ready are of level L.
+template <class Gp, class GetF>
+__device__ __forceinline__ void expand(const Gp& g, const LvArgs& a, const LvLists& ls, int m,
+                                       int at, int threads, int L, GetF get) {
+  const int lane = threadIdx.x & 31;
+  for (int i0 = at & ~31; i0 < 4 * m; i0 += threads) {
+    const int i = i0 + lane;
+    int x = i < 4 * m ? get(i >> 2, i & 3) : -1;
+    if (__any_sync(FULL, x == kWide)) {  // only a record's last word is kWide
+      const bool wide = __shfl_sync(FULL, x, lane | 3) == kWide;
+      const int e0 = __shfl_sync(FULL, x, lane & ~3), deg = __shfl_sync(FULL, x, (lane & ~3) | 1);
+      if (wide) x = deg <= kWideMax && (lane & 3) < deg ? a.fanin[e0 + (lane & 3)] : -1;
+      unsigned todo = __ballot_sync(FULL, wide && deg > kWideMax && (lane & 3) == 0);
+      while (todo) {  // a warp at a time
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int e1 = __shfl_sync(FULL, e0, src), d1 = __shfl_sync(FULL, deg, src);
+        for (int e = 0; e < d1; e += 32)
+          decrement(g, a, ls, e + lane < d1 ? a.fanin[e1 + e + lane] : -1, L);
+      }
+    }
+    decrement(g, a, ls, x, L);
+  }
+}
+
+// The seed: order and level 0, their counters out of reach of decrements.
+template <class Gp>
+__device__ __forceinline__ void seed(const Gp& g, const LvArgs& a, int at, int threads) {
+  for (int k = at; k < a.first_size; k += threads) {
+    const int v = a.frontier0[k];
+    a.order[k] = v;
+    if ((unsigned)v < (unsigned)a.n) {
+      a.level[v] = 0;
+      *g.counter(v) = INT_MAX;
+    } else {
+      atomicCAS(&a.ctl->grid.status, 0, (int)OTG_ERR_INVALID);
+    }
+  }
+}
+__device__ __forceinline__ int seed_word(const LvArgs& a, int k, int f) {
+  const int u = a.frontier0[k];
+  return (unsigned)u < (unsigned)a.n ? ((const int*)a.packed)[4 * (size_t)u + f] : -1;
+}
+__device__ __forceinline__ int spill_word(const LvArgs& a, int L, int k, int f) {
+  const int u = __ldcg(a.spill + (size_t)(L & 1) * a.n + k);
+  return __ldcg((const int*)a.packed + 4 * (size_t)u + f);
+}
+
+// ---- the cluster form ----------------------------------------------------
+//
+// Pin v's counter lies in CTA v mod S (neighbouring pins are often of one
+// level, so ranges would send a level's atomics to one CTA).  A CTA that
+// readied more than kLocalMax entries of a level hands the rest to a CTA
+// chosen by a hash of the pin (a buffer tree readies its levels from one
+// place); what no list holds goes to the spill list in global memory.  Two
+// warps write the pins' levels and fetch the CTAs' list lengths, and find
+// the end one level late: 16 stores from each CTA into all others cost 600
+// cycles of the barrier that waits for them, and a global store 400.
+//
+// No wait here polls memory: the cluster barrier is hardware, and every CTA
+// takes the same number of barriers (the loop ends on lengths that every
+// CTA reads alike).
+constexpr int kLocalMax = 64;
+constexpr int kNoteWarps = 2;
+
+struct ClWords {
+  int len[4];  // list lengths by level (may exceed the capacity); a level's is filled in the
+               // level before, read in its own, cleared in the next
+  int ovf[4];  // some pin of the level was spilled (set in every CTA)
+  int done;    // an empty level was reached
+};
+
+struct ClGroup {
+  const cg::cluster_group& cl;
+  const LvArgs& a;
+  const LvLists& ls;
+  ClWords& sw;
+  int* scnt;   // this CTA's counters, or null: the global ones
+  int sshift;  // log2 of the cluster size
+  __device__ int* counter(int v) const {
+    return scnt ? cl.map_shared_rank(scnt + (v >> sshift), v & ((1 << sshift) - 1)) : a.cnt + v;
+  }
+  __device__ int* length(int L) const { return &sw.len[L & 3]; }
+  __device__ int most() const { return kLocalMax; }
+  __device__ void spill(int v, int L) const {
+    spill_pin(a, v, L);
+    for (int i = 0; i < (1 << sshift); ++i) *cl.map_shared_rank(&sw.ovf[L & 3], i) = 1;
+  }
+  __device__ void hand_on(int v, int4 pk, int recs, int L) const {
+    const int t = sshift ? (int)(((unsigned)v * 0x9E3779B1u) >> (32 - sshift)) : 0;
+    const int at = atomicAdd(cl.map_shared_rank(&sw.len[L & 3], t), recs);
+    if (!put_records(cl.map_shared_rank(ls.rec(L), t), cl.map_shared_rank(ls.pin(L), t), ls.cap,
+                     at, recs, v, pk))
+      spill(v, L);
+  }
+};
 
 template <int CT>
-__global__ void __launch_bounds__(CT, 1) levelize_cluster_kernel(
-    int n, const int* fanin_start, const int* fanin, const int* out_deg, const int* frontier0,
-    int first_size, int* order, int* level, int* level_ends, int* counts, LvCtl* ctl, int* cnt,
-    int cshift, int lst_cap, int scnt_on) {
-  const int C = 1 << cshift;  // bitmap words per CTA range
-  extern __shared__ unsigned lv_sm[];
-  unsigned* const bm0 = lv_sm;  // level L's ready pins: bm0 for even L, bm1 for odd
-  unsigned* const bm1 = lv_sm + C;
-  // with scnt_on: the fanin counters of the range's 32*C pins
-  int* const scnt = scnt_on ? (int*)(lv_sm + 2 * C) : nullptr;
-  // fanin ranges to expand at even / odd levels
-  int2* const lst0 = (int2*)(lv_sm + 2 * C + (scnt_on ? 32 * C : 0));
-  int2* const lst1 = lst0 + lst_cap;
-  // per-level scalars in three rotating slots (this level, the next, the
-  // one after): a slot is cleared a level before anything adds to it, so
-  // no block barrier orders the clear
-  __shared__ int rc[3][16];  // ready pins of every CTA's range (each CTA keeps a copy)
-  __shared__ int lcnt[3];  // length of the list of fanin ranges
-  __shared__ int ovf[3];   // some CTA's list overflowed
-  __shared__ int wsum[2][2 * (CT / 32)];  // warp totals of the level's scans, by level parity
-  __shared__ int s_excl[CT], s_e0[CT];    // list entries: warp-exclusive edge start, fanin start
+__global__ void __launch_bounds__(CT, 1)
+    levelize_cluster_kernel(LvArgs a, int lst_cap, int scnt_on) {
+  extern __shared__ __align__(16) unsigned lv_sm[];
+  __shared__ ClWords sw;
   const cg::cluster_group cl = cg::this_cluster();
   const int S = (int)cl.num_blocks(), r = (int)cl.block_rank(), tid = threadIdx.x;
-  const int sshift = 31 - __clz(S);  // cluster sizes are powers of two
-  const int gtid = r * CT + tid, gstride = S * CT;
-  const int nw = (n + 31) >> 5;
-  const int lane = tid & 31, w = tid >> 5;
-
-  for (int v = gtid; v < n; v += gstride) {
-    if (!scnt) cnt[v] = out_deg[v];
-    level[v] = -1;
-  }
-  if (scnt)
-    for (int j = tid; j < 32 * C; j += CT) {
-      const int v = (r << (cshift + 5)) + j;
-      scnt[j] = v < n ? out_deg[v] : 0;
-    }
-  for (int i = tid; i < 2 * C; i += CT) lv_sm[i] = 0u;
-  if (tid < 48) rc[tid / 16][tid % 16] = 0;
-  if (tid < 3) { lcnt[tid] = 0; ovf[tid] = 0; }
+  const int gtid = r * CT + tid, gstride = S * CT, lane = tid & 31;
+  const LvLists ls{(int4*)lv_sm, (int*)((int4*)lv_sm + 2 * lst_cap), lst_cap};
+  const ClGroup g{cl, a, ls, sw, scnt_on ? ls.pin0 + 2 * lst_cap : nullptr, 31 - __clz(S)};
+  if (g.scnt)
+    for (int v = r + tid * S; v < a.n; v += CT * S) g.scnt[v >> g.sshift] = a.out_deg[v];
+  if (tid < (int)(sizeof(ClWords) / 4)) ((int*)&sw)[tid] = 0;
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the records, counters and levels' fill
   cl.sync();
-  for (int k = gtid; k < first_size; k += gstride) {
-    const int v = frontier0[k];
-    order[k] = v;
-    if ((unsigned)v < (unsigned)n) {
-      level[v] = 0;
-      // after the counters' fill (cluster barrier above)
-      if (scnt) {
-        const int owner = v >> (cshift + 5);
-        *cl.map_shared_rank(scnt + (v - (owner << (cshift + 5))), owner) = INT_MAX;
-      } else {
-        cnt[v] = INT_MAX;
-      }
-    } else {
-      atomicCAS(&ctl->status, 0, (int)OTG_ERR_INVALID);
-    }
-  }
-  if (gtid == 0) {
-    level_ends[0] = 0;
-    if (first_size > 0) level_ends[1] = first_size;
-  }
-  if (first_size == 0) {  // uniform: no CTA has touched another's memory
-    if (gtid == 0) { counts[0] = 0; counts[1] = 0; }
-    return;
-  }
+  seed(g, a, gtid, gstride);
   cl.sync();
-  // expand the seed into level 1 (bm1, slot 1, lst1)
-  {
-    const ClNext nx{bm1, scnt, cshift, sshift, rc[1], lst1, &lcnt[1], &ovf[1], lst_cap};
-    for (int k0 = r * CT; k0 < first_size; k0 += gstride) {
-      const int k = k0 + tid;
-      const bool act = k < first_size && (unsigned)order[k] < (unsigned)n;
-      const int u = act ? order[k] : 0;
-      int e = act ? fanin_start[u] : 0;
-      const int e1 = act ? fanin_start[u + 1] : 0;
-      while (__any_sync(FULL, e < e1)) {
-        const bool has = e < e1;
-        const int v = has ? fanin[e] : -1;
-        decrement_cl(v, has && (unsigned)v < (unsigned)n, fanin_start, cnt, nx, cl);
-        e += has ? 1 : 0;
-      }
-    }
-  }
-  int emitted = first_size;
+  expand(g, a, ls, a.first_size, gtid, gstride, 1, [&](int k, int f) { return seed_word(a, k, f); });
+  constexpr int XT = CT - 32 * kNoteWarps;  // expanding threads
   int L = 1;
-  const int w0 = min(nw, r * C), w1 = min(nw, (r + 1) * C);
-  // this thread's words of the range: KW consecutive ones
-  const int KW = max(1, (w1 - w0 + CT - 1) / CT);
-  const int i0 = min(w1, w0 + tid * KW), i1 = min(w1, i0 + KW);
-  int q_now = 1, q_next = 2, q_free = 0;
-  LV_PHASE_BEGIN();
-  while (true) {
+  for (;; ++L) {
     cl.sync();
-    LV_PHASE(0);
-    const int par = L & 1;
-    unsigned* cur = par ? bm1 : bm0;
-    int2* lcur = par ? lst1 : lst0;
-    const ClNext nx{par ? bm0 : bm1,   scnt,          cshift,       sshift, rc[q_next],
-                    par ? lst0 : lst1, &lcnt[q_next], &ovf[q_next], lst_cap};
-    if (tid < 16) rc[q_free][tid] = 0;  // read a level ago; added to from the next level on
-    if (tid == 0) {
-      lcnt[q_free] = 0;
-      ovf[q_free] = 0;
-    }
-    // every warp: the level total and this CTA's offset from the counts
-    const int x = lane < S ? rc[q_now][lane] : 0;
-    const int before = __reduce_add_sync(FULL, lane < r ? x : 0);
-    const int total = __reduce_add_sync(FULL, x);
-    if (total == 0) break;  // uniform: every CTA read the same counts
-    const int run = emitted + before;
-    const int m = lcnt[q_now];          // appended before the cluster barrier
-    const bool over = ovf[q_now] != 0;  // likewise; the same in every CTA
-#ifdef OTG_PHASE_TIMING
-    if (tid == 0 && L < 4096) counts[16 + L * 16 + r] = m;
-    const long long _lt0 = clock64();
-#endif
-    LV_PHASE(3);
-    // the emission writes the range's pins in ascending order into `order`
-    // with their level and clears the words for reuse two levels on
-    auto emit = [&](int pos) {
-      for (int i = i0; i < i1; ++i) {
-        unsigned bits = cur[i - r * C];
-        while (bits) {
-          const int bit = __ffs(bits) - 1;
-          bits &= bits - 1;
-          const int v = (i << 5) + bit;
-          if (pos < n) order[pos] = v;
-          else atomicCAS(&ctl->status, 0, (int)OTG_ERR_INVALID);  // duplicate seeds
-          ++pos;
-          level[v] = L;
-        }
-        cur[i - r * C] = 0u;
+    if (sw.done) break;
+    const int p = L & 1, m = min(sw.len[L & 3], ls.cap);
+    const bool over = sw.ovf[L & 3] != 0;
+    if (tid < XT) {
+      const int4* rec = ls.rec(L);
+      expand(g, a, ls, m, tid, XT, L + 1, [&](int k, int f) { return ((const int*)(rec + k))[f]; });
+      if (over) {
+        const int ns = __ldcg(&a.ctl->spill[L & 3]);
+        for (int k = r * XT + tid; k < ns; k += S * XT) a.level[__ldcg(a.spill + (size_t)p * a.n + k)] = L;
+        expand(g, a, ls, ns, r * XT + tid, S * XT, L + 1,
+               [&](int k, int f) { return spill_word(a, L, k, f); });
       }
-    };
-    int pc = 0;
-    for (int i = i0; i < i1; ++i) pc += __popc(cur[i - r * C]);
-    constexpr int W = CT / 32;
-    // Expansion of fanin ranges range(k), k < mm, CT at a time: ONE block
-    // scan per chunk hands one edge to each thread -- an edge q finds its
-    // warp by a shuffle search over the warps' edge totals, then its range
-    // by a binary search over that warp's exclusive starts.  With `emit_on`
-    // the first chunk's scan also gives the emission offsets (popcounts),
-    // and the emission runs while the first fanin loads are in flight.
-    auto expand = [&](int mm, auto range, bool emit_on) {
-      bool pending = emit_on;
-      int c0 = 0;
-      do {
-        const int k = c0 + tid;
-        const int2 en = k < mm ? range(k) : make_int2(0, 0);
-        int y1 = en.y, y2 = (emit_on && c0 == 0) ? pc : 0;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int z1 = __shfl_up_sync(FULL, y1, d), z2 = __shfl_up_sync(FULL, y2, d);
-          if (lane >= d) {
-            y1 += z1;
-            y2 += z2;
-          }
-        }
-        s_excl[tid] = y1 - en.y;
-        s_e0[tid] = en.x;
-        if (lane == 31) {
-          wsum[par][w] = y1;
-          wsum[par][W + w] = y2;
-        }
-        __syncthreads();
-        const int tE = lane < W ? wsum[par][lane] : 0;
-        const int tP = lane < W ? wsum[par][W + lane] : 0;
-        const int epos = run + __reduce_add_sync(FULL, lane < w ? tP : 0) + y2 - pc;
-        int inclE = tE;  // lane u: edges of warps 0..u
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int z = __shfl_up_sync(FULL, inclE, d);
-          if (lane >= d) inclE += z;
-        }
-        const int etot = __shfl_sync(FULL, inclE, 31);
-        for (int q0 = 0; q0 < etot; q0 += CT) {
-          const int q = q0 + tid;
-          const int qc = min(q, etot - 1);  // every lane searches (the shuffles are warp-wide)
-          int u = 0;                        // warps whose edges all lie before qc
-#pragma unroll
-          for (int step = 16; step >= 1; step >>= 1) {
-            const int ic = __shfl_sync(FULL, inclE, (u + step - 1) & 31);
-            if (ic <= qc) u += step;
-          }
-          const int base = __shfl_sync(FULL, inclE, (u - 1) & 31);
-          const int ql = qc - (u > 0 ? base : 0);
-          const int* xs = s_excl + u * 32;
-          int j = 0;  // the last range of warp u whose start is <= ql
-#pragma unroll
-          for (int step = 16; step >= 1; step >>= 1)
-            if (xs[j + step] <= ql) j += step;
-          const int v = q < etot ? fanin[s_e0[u * 32 + j] + (ql - xs[j])] : -1;
-          if (pending) {
-            emit(epos);
-            pending = false;
-          }
-          decrement_cl(v, (unsigned)v < (unsigned)n, fanin_start, cnt, nx, cl);
-        }
-        if (pending) {
-          emit(epos);
-          pending = false;
-        }
-        c0 += CT;
-        if (c0 < mm) __syncthreads();  // the next chunk reuses s_excl, s_e0 and wsum
-      } while (c0 < mm);
-    };
-    if (!over) {
-      // the fanin ranges this CTA collected last level
-      expand(m, [&](int k) { return lcur[k]; }, true);
-      LV_PHASE(1);
     } else {
-      // a list overflowed last level: every CTA emits its own range's pins
-      // of this level and expands them, read back from `order`, their
-      // fanin ranges from global memory
-      int y2 = pc;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int z2 = __shfl_up_sync(FULL, y2, d);
-        if (lane >= d) y2 += z2;
+      const int x = lane < S ? *(volatile int*)cl.map_shared_rank(&sw.len[L & 3], lane) : 0;
+      for (int k = tid - XT; k < m; k += 32 * kNoteWarps) {
+        const int v = ls.pin(L)[k];
+        if (v >= 0) a.level[v] = L;
       }
-      if (lane == 31) wsum[par][W + w] = y2;
-      __syncthreads();
-      const int tP = lane < W ? wsum[par][W + lane] : 0;
-      const int wbP = __reduce_add_sync(FULL, lane < w ? tP : 0);
-      const int tt = min(__reduce_add_sync(FULL, tP), n - run);
-      emit(run + wbP + y2 - pc);
-      __syncthreads();  // this range's slice of `order` is written; wsum is reused
-      expand(
-          tt,
-          [&](int k) {
-            const int u = __ldcg(order + run + k);
-            const int e0 = fanin_start[u];
-            return make_int2(e0, fanin_start[u + 1] - e0);
-          },
-          false);
+      if (!__any_sync(FULL, x != 0) && !over && lane == 0) sw.done = 1;
     }
-    emitted += total;
-    if (emitted > n) {  // only reachable with duplicate seeds; stop cleanly
-      if (gtid == 0) atomicCAS(&ctl->status, 0, (int)OTG_ERR_INVALID);
-      emitted = n;
-      break;
+    // the level before this one is behind every CTA
+    if (tid == 0) {
+      sw.len[(L - 1) & 3] = sw.ovf[(L - 1) & 3] = 0;
+      if (r == 0) a.ctl->spill[(L - 1) & 3] = 0;
     }
-    if (gtid == 0) level_ends[L + 1] = emitted;
-#ifdef OTG_PHASE_TIMING
-    if (tid == 0 && L < 4096) counts[16 + 65536 + L * 16 + r] = (int)(clock64() - _lt0);
-#endif
-    ++L;
-    const int q = q_free;
-    q_free = q_now;
-    q_now = q_next;
-    q_next = q;
-    LV_PHASE(2);
   }
-  if (gtid == 0) {
-    counts[0] = L;
-    counts[1] = emitted;
-  }
-  LV_PHASE_END(counts);
-  cl.sync();  // no CTA leaves while another may still read its counts
+  if (gtid == 0) a.ctl->levels = L - 1;
+  cl.sync();  // no CTA leaves while another may still read its list length
 }
 
-// Dynamic shared memory of the cluster path: both bitmaps (C words each),
-// optionally the range's fanin counters (32*C ints), and two lists of at
-// least kLstMin fanin ranges (8 bytes each); the lists take what is left of
-// kClusterSmemMax.
+// ---- the grid form -------------------------------------------------------
+//
+// A CTA per SM.  A CTA that has readied a quarter more than its share of a
+// level's entries, going by the level before, puts further pins on the
+// spill list, which all CTAs share out: the CTAs with the most pins ready
+// the most, so that lists left alone drift apart (68 to 558 entries on
+// average over 5M pins' 200 levels).
+constexpr int LT = 1024;
+constexpr int kGridCap = 4096, kGridLeast = 64;
+constexpr int kSpillWarps = 4;  // the warps that take the CTA's share of the spill list
+
+// A grid barrier for many uses in one launch: arrivals only count up, so the
+// last CTA's arrival is itself what the others wait for (a counter that is
+// reset and a generation that is then raised, each behind a fence, took
+// 4.5 us a level).  Waits are bounded as grid_barrier's.
+struct GridWait {
+  GridCtl* c;
+  unsigned target = 0;
+  __device__ bool wait() {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&c->count) : "memory");
+      target += gridDim.x;
+      int ok = 1;
+      unsigned long long t0 = 0;
+      for (int k = 0;; ++k) {
+        unsigned v;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&c->count) : "memory");
+        if ((int)(v - target) >= 0) break;
+        if ((k & 15) != 15) continue;
+        const unsigned long long t = gtime();
+        if (t0 == 0) t0 = t;
+        if (t - t0 > kGridWaitNs) {
+          atomicExch(&c->abort, 1);
+          atomicCAS(&c->status, 0, (int)OTG_ERR_TIMEOUT);
+        }
+        if (*(volatile int*)&c->abort) {
+          ok = 0;
+          break;
+        }
+      }
+      s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+  }
+};
+
+struct GridGroup {
+  const LvArgs& a;
+  int* len;         // by level parity
+  const int* room;  // entries before a warp puts pins on the spill list
+  __device__ int* counter(int v) const { return a.cnt + v; }
+  __device__ int* length(int L) const { return len + (L & 1); }
+  __device__ int most() const { return *room; }
+  __device__ void spill(int v, int L) const { spill_pin(a, v, L); }
+  __device__ void hand_on(int v, int4, int, int L) const { spill_pin(a, v, L); }
+};
+
+__global__ void __launch_bounds__(LT, 1) levelize_grid_kernel(LvArgs a) {
+  extern __shared__ __align__(16) unsigned lv_sm[];
+  __shared__ int s_len[2], s_room, s_done;
+  const int G = gridDim.x, tid = threadIdx.x;
+  const int gtid = blockIdx.x * LT + tid, gstride = G * LT;
+  const LvLists ls{(int4*)lv_sm, (int*)((int4*)lv_sm + 2 * kGridCap), kGridCap};
+  const GridGroup g{a, s_len, &s_room};
+  GridWait barrier{&a.ctl->grid};
+  if (tid < 2) s_len[tid] = 0;
+  if (tid == 0) {
+    s_room = max(kGridLeast, a.first_size / G);
+    s_done = 0;
+  }
+  seed(g, a, gtid, gstride);
+  if (!barrier.wait()) return;
+  expand(g, a, ls, a.first_size, gtid, gstride, 1, [&](int k, int f) { return seed_word(a, k, f); });
+  constexpr int XT = LT - 32 * kSpillWarps;  // the threads of the CTA's own list
+  int L = 1;
+  for (;; ++L) {
+    const int p = L & 1;
+    __syncthreads();
+    if (tid == 0 && s_len[p]) atomicAdd(&a.ctl->tot[L & 3], s_len[p]);
+    if (!barrier.wait()) return;
+    if (s_done) break;  // the same in every CTA: all read the same totals
+    const int m = min(s_len[p], ls.cap);
+    if (tid < XT) {
+      for (int k = tid; k < m; k += XT) {
+        const int v = ls.pin(L)[k];
+        if (v >= 0) a.level[v] = L;
+      }
+      const int4* rec = ls.rec(L);
+      expand(g, a, ls, m, tid, XT, L + 1, [&](int k, int f) { return ((const int*)(rec + k))[f]; });
+    } else {
+      // the level's totals (nobody else waits for them: the end is found a
+      // level late), and every G-th pin of the spill list
+      const int tot = __ldcg(&a.ctl->tot[L & 3]), ns = __ldcg(&a.ctl->spill[L & 3]);
+      if (tid == XT) {
+        if (tot == 0 && ns == 0) s_done = 1;
+        s_room = max(kGridLeast, min((int)((long long)(tot + ns) * 5 / 4 / G), kGridCap / 2));
+      }
+      const int b = blockIdx.x, share = max(0, (ns - b + G - 1) / G);
+      for (int k = tid - XT; k < share; k += LT - XT)
+        a.level[__ldcg(a.spill + (size_t)p * a.n + b + k * G)] = L;
+      expand(g, a, ls, share, tid - XT, LT - XT, L + 1,
+             [&](int k, int f) { return spill_word(a, L, b + k * G, f); });
+    }
+    __syncthreads();
+    if (tid == 0) {
+      s_len[p] = 0;  // level L + 2's
+      if (blockIdx.x == 0) a.ctl->tot[(L - 1) & 3] = a.ctl->spill[(L - 1) & 3] = 0;
+    }
+  }
+  if (gtid == 0) a.ctl->levels = L - 1;
+}
+
+// ---- the sort ------------------------------------------------------------
+//
+// Pins by level - 1 (level 0 is the seed, in the caller's order), stable in
+// the pin index: digits of kDigitBits, each by a histogram per tile of
+// consecutive items, a scan and a scatter.  Graphs of more than kDigits + 1
+// levels take a second digit, whose kernels return at once otherwise.
+constexpr int kDigitBits = 10, kDigits = 1 << kDigitBits, kMaxTiles = 256, ST = 1024;
+
+struct LvSort {
+  int per;      // items per tile
+  int tiles;
+  int* hist;    // [kDigits][tiles]
+  int* first;   // the pins by the first digit, where there are two
+  int* num;     // their number
+};
+
+// Item i of a pass and its digit (-1: not an item): the pins in index order
+// (pass 0), or the first pass's output.
+__device__ __forceinline__ int sort_item(const LvArgs& a, const LvSort& s, int pass, int i,
+                                         int& v) {
+  if (pass == 0) {
+    v = i;
+    const int l = i < a.n ? a.level[i] : 0;
+    return l > 0 ? (l - 1) & (kDigits - 1) : -1;
+  }
+  if (i >= *s.num) return -1;
+  v = s.first[i];
+  return ((a.level[v] - 1) >> kDigitBits) & (kDigits - 1);
+}
+__device__ __forceinline__ bool sort_skip(const LvArgs& a, int pass) {
+  return pass == 1 && a.ctl->levels <= kDigits + 1;
+}
+
+__global__ void __launch_bounds__(ST) levelize_hist(LvArgs a, LvSort s, int pass) {
+  __shared__ int h[kDigits];
+  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
+  if (sort_skip(a, pass)) return;
+  for (int d = threadIdx.x; d < kDigits; d += ST) h[d] = 0;
+  __syncthreads();
+  const int b = blockIdx.x * s.per;
+  for (int i = threadIdx.x; i < s.per; i += ST) {
+    int v;
+    const int d = sort_item(a, s, pass, b + i, v);
+    if (d >= 0) atomicAdd(&h[d], 1);
+  }
+  __syncthreads();
+  for (int d = threadIdx.x; d < kDigits; d += ST) s.hist[d * s.tiles + blockIdx.x] = h[d];
+}
+
+// Exclusive scan over (digit, tile), a thread per digit; with one digit, the
+// levels' ends and the counts too.
+__global__ void __launch_bounds__(kDigits) levelize_scan(LvArgs a, LvSort s, int pass) {
+  __shared__ int wsum[kDigits / 32];
+  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
+  if (sort_skip(a, pass)) return;
+  const int d = threadIdx.x, lane = d & 31, w = d >> 5;
+  int* row = s.hist + d * s.tiles;
+  int sum = 0;
+#pragma unroll 8
+  for (int t = 0; t < s.tiles; ++t) sum += row[t];
+  int x = sum;
+#pragma unroll
+  for (int k = 1; k < 32; k <<= 1) {
+    const int y = __shfl_up_sync(FULL, x, k);
+    if (lane >= k) x += y;
+  }
+  if (lane == 31) wsum[w] = x;
+  __syncthreads();
+  const int below = wsum[lane];
+  int run = __reduce_add_sync(FULL, lane < w ? below : 0) + x - sum;
+  const int total = __reduce_add_sync(FULL, below);
+  const int levels = a.ctl->levels, end = a.first_size + run + sum;
+#pragma unroll 8
+  for (int t = 0; t < s.tiles; ++t) {
+    const int c = row[t];
+    row[t] = run;
+    run += c;
+  }
+  if (pass == 0 && d + 1 < levels) a.level_ends[d + 2] = min(end, a.n);
+  if (pass == 0 && d == 0) {
+    *s.num = total;
+    a.level_ends[0] = 0;
+    if (levels > 0) a.level_ends[1] = a.first_size;
+    // only with duplicate seeds are there more than n
+    if (a.first_size + total > a.n) atomicCAS(&a.ctl->grid.status, 0, (int)OTG_ERR_INVALID);
+    a.counts[0] = levels;
+    a.counts[1] = min(a.first_size + total, a.n);
+  }
+}
+
+// The lanes with the same digit (d < 0: none), bit by bit; see decrement on
+// match_any.
+__device__ __forceinline__ unsigned same_digit(int d) {
+  unsigned peers = __ballot_sync(FULL, d >= 0);
+#pragma unroll
+  for (int k = 0; k < kDigitBits; ++k) {
+    const unsigned on = __ballot_sync(FULL, (d >> k) & 1);
+    peers &= (d >> k) & 1 ? on : ~on;
+  }
+  return peers;
+}
+
+__global__ void __launch_bounds__(ST) levelize_scatter(LvArgs a, LvSort s, int pass) {
+  extern __shared__ __align__(16) unsigned lv_sm[];
+  uint16_t* cnt = (uint16_t*)lv_sm;                  // [warp][digit], then the warps' bases
+  int* base = (int*)(cnt + (ST / 32) * kDigits);     // [digit] the tile's base
+  asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
+  if (sort_skip(a, pass)) return;
+  const bool last = pass == 1 || a.ctl->levels <= kDigits + 1;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int i = threadIdx.x; i < (ST / 32) * kDigits / 2; i += ST) ((unsigned*)cnt)[i] = 0u;
+  for (int d = threadIdx.x; d < kDigits; d += ST) base[d] = s.hist[d * s.tiles + blockIdx.x];
+  __syncthreads();
+  // each warp takes consecutive items, 32 at a time
+  const int per = s.per / (ST / 32), b = blockIdx.x * s.per + w * per;
+  uint16_t* mine = cnt + w * kDigits;
+  for (int i = 0; i < per; i += 32) {
+    int v;
+    const int d = sort_item(a, s, pass, b + i + lane, v);
+    const unsigned peers = same_digit(d);
+    if (d >= 0 && __ffs(peers) - 1 == lane) mine[d] += (uint16_t)__popc(peers);
+    __syncwarp();
+  }
+  __syncthreads();
+  for (int d = threadIdx.x; d < kDigits; d += ST) {
+    int run = 0;
+#pragma unroll 8
+    for (int k = 0; k < ST / 32; ++k) {
+      const int c = cnt[k * kDigits + d];
+      cnt[k * kDigits + d] = (uint16_t)run;
+      run += c;
+    }
+  }
+  __syncthreads();
+  int* out = last ? a.order : s.first;
+  const int off = last ? a.first_size : 0;
+  for (int i = 0; i < per; i += 32) {
+    int v;
+    const int d = sort_item(a, s, pass, b + i + lane, v);
+    const unsigned peers = same_digit(d);
+    int pos = 0;
+    if (d >= 0) pos = off + base[d] + mine[d] + __popc(peers & ((1u << lane) - 1u));
+    __syncwarp();
+    if (d >= 0) {
+      if (__ffs(peers) - 1 == lane) mine[d] += (uint16_t)__popc(peers);
+      if (pos < a.n) out[pos] = v;
+    }
+    __syncwarp();
+  }
+}
+
+// The levels' ends from the sorted pins, where the first digit did not give
+// them.
+__global__ void levelize_ends(LvArgs a, LvSort s) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (sort_skip(a, 1)) return;
+  const int end = min(a.first_size + *s.num, a.n);
+  for (int p = a.first_size + blockIdx.x * blockDim.x + threadIdx.x; p < end;
+       p += gridDim.x * blockDim.x) {
+    const int l = a.level[a.order[p]];
+    if (p == a.first_size || a.level[a.order[p - 1]] != l) a.level_ends[l] = p;
+    if (p == end - 1) a.level_ends[l + 1] = end;
+  }
+}
+
+// ---- host ------------------------------------------------------------------
 constexpr size_t kClusterSmemMax = 200 * 1024;
-constexpr int kLstMin = kCtMax;
-size_t lv_cluster_smem(int C, bool scnt) {
-  return (size_t)(2 * C + (scnt ? 32 * C : 0) + 4 * kLstMin) * 4;
-}
-int lv_lst_cap(int C, bool scnt) {
-  return ((int)(kClusterSmemMax / 4) - 2 * C - (scnt ? 32 * C : 0)) / 4;
-}
+constexpr int kLstMin = 1024;  // entries of a CTA's list at least
+constexpr size_t kEntry = 2 * (sizeof(int4) + sizeof(int));
+size_t scnt_bytes(int n, int S) { return 4 * (((size_t)n + S - 1) / S); }
 
 constexpr int kWidths[4] = {128, 256, 512, 1024};
 const void* cluster_fn(int wi) {
@@ -690,10 +622,11 @@ const void* cluster_fn(int wi) {
     default: return (const void*)levelize_cluster_kernel<1024>;
   }
 }
+constexpr size_t kGridSmem = kEntry * kGridCap;
+constexpr size_t kScatterSmem = 2 * (ST / 32) * kDigits + 4 * kDigits;
 
 struct LvDev {
   int sms = 0;
-  int occ = 0;
   bool init = false;
   int max_cluster[4] = {0, 0, 0, 0};  // per CTA width: largest cluster (power of two <= 16) placed
 };
@@ -705,8 +638,10 @@ LvDev& lv_dev() {
   LvDev& x = g_lv[d & 63];
   if (!x.init) {
     cudaDeviceGetAttribute(&x.sms, cudaDevAttrMultiProcessorCount, d);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&x.occ, levelize_kernel, LT, 0);
-    x.occ = std::max(1, std::min(x.occ, 2));
+    cudaFuncSetAttribute(levelize_grid_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kGridSmem);
+    cudaFuncSetAttribute(levelize_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)kScatterSmem);
     // the cluster path: allow its largest shared memory and 16-CTA clusters,
     // then keep, per CTA width, the largest cluster size the device places
     for (int wi = 0; wi < 4; ++wi) {
@@ -739,24 +674,26 @@ LvDev& lv_dev() {
   return x;
 }
 
-// The cluster path's shape for an n-pin graph: S CTAs of kWidths[wi]
-// threads, each owning 2^cshift bitmap words.  S = 0: the cooperative path.
+// The cluster form's shape for an n-pin graph: S CTAs of kWidths[wi]
+// threads.  S = 0: the grid form.
 struct ClPlan {
-  int S = 0, wi = 0, cshift = 0;
-  bool scnt = false;  // the fanin counters in shared memory
+  int S = 0, wi = 0, cap = 0;
+  bool scnt = false;  // the fanout counters in shared memory
 };
-// Default: the largest cluster the device places (16 CTAs on B200) of 256
-// threads each, for graphs whose ranges then hold at most kClusterMaxWords
-// words (about a million pins); larger graphs take the cooperative path,
-// which spreads a level over every SM.  OTG_LEVELIZE_CLUSTER=0 turns the
-// cluster path off, =1|2|4|8|16 asks for that size; OTG_LEVELIZE_CT=
-// 128|256|512|1024 asks for that width (both only where the graph fits and
-// the device places the cluster).
-constexpr int kClusterMaxWords = 2048;
+// Default: the largest cluster the device places (16 CTAs on B200) of 512
+// threads each, for graphs whose counters it holds (up to 650k pins); larger
+// graphs take the grid form, which spreads a level over every SM.  Cluster
+// against grid: 163k pins / 374 levels 551 and 1053 us, 400k / 200 levels 593
+// and 687, 329k / 106 levels 400 and 403; with the counters in global memory
+// 900k / 300 levels 1289 and 1137.  256 threads take 712, 861 and 539 us on
+// the first three (fewer warps expand), 1024 602 on the first.
+// OTG_LEVELIZE_CLUSTER=0 turns the cluster form off, =1|2|4|8|16 asks for
+// that size; OTG_LEVELIZE_CT=128|256|512|1024 asks for that width (both only
+// where the device places the cluster); OTG_LEVELIZE_SCNT=0 keeps the
+// counters in global memory.
 ClPlan lv_cluster_plan(int n, const LvDev& d) {
   ClPlan p;
-  const int nw = std::max(1, (n + 31) / 32);
-  p.wi = 1;
+  p.wi = 2;
   if (const char* e = std::getenv("OTG_LEVELIZE_CT")) {
     const int want = std::atoi(e);
     for (int wi = 0; wi < 4; ++wi)
@@ -770,39 +707,63 @@ ClPlan lv_cluster_plan(int n, const LvDev& d) {
     if (want <= 0) return ClPlan{};
     s = 1;
     while (s < want && s < maxc) s <<= 1;
-  } else if ((nw + s - 1) / s > kClusterMaxWords) {
-    return ClPlan{};  // large graphs: the whole GPU (the cooperative path)
+  } else if (scnt_bytes(n, s) + kEntry * kLstMin > kClusterSmemMax) {
+    return ClPlan{};
   }
-  int cs = 0;
-  while ((1 << cs) * s < nw) ++cs;
-  if (lv_cluster_smem(1 << cs, false) > kClusterSmemMax) return ClPlan{};
   p.S = s;
-  p.cshift = cs;
-  // the counters go on chip where they fit (ranges of up to 32k pins:
-  // graphs of about half a million pins); OTG_LEVELIZE_SCNT=0 keeps them in
-  // global memory
-  p.scnt = lv_cluster_smem(1 << cs, true) <= kClusterSmemMax;
+  p.scnt = scnt_bytes(n, s) + kEntry * kLstMin <= kClusterSmemMax;
   if (const char* e = std::getenv("OTG_LEVELIZE_SCNT"))
     if (std::atoi(e) == 0) p.scnt = false;
+  p.cap = (int)((kClusterSmemMax - (p.scnt ? scnt_bytes(n, s) : 0)) / kEntry) & ~3;
   return p;
 }
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
+// Items per sort tile: a multiple of 32 per warp, about kMaxTiles tiles at
+// most, and no more than the scatter's 16-bit counts hold.
+LvSort lv_tiles(int n) {
+  LvSort s{};
+  s.per = 8 * ST;
+  while (s.per < 63 * ST && (long long)s.per * kMaxTiles < n) s.per += ST;
+  s.tiles = std::max(1, (int)(((long long)n + s.per - 1) / s.per));
+  return s;
+}
+
 struct LvWs {
-  size_t ctl, cnt, bm0, bm1, blk, total;
+  size_t ctl, cnt, packed, spill, hist, total;
 };
-LvWs lv_ws(int n, int G) {
+LvWs lv_ws(int n) {
   LvWs l;
+  const size_t N = (size_t)std::max(n, 1);
   size_t o = 0;
-  l.ctl = o; o = align256(o + sizeof(LvCtl));
-  l.cnt = o; o = align256(o + 4 * (size_t)std::max(n, 1));
-  const size_t nw = ((size_t)n + 31) / 32 + 1;
-  l.bm0 = o; o = align256(o + 4 * nw);
-  l.bm1 = o; o = align256(o + 4 * nw);
-  l.blk = o; o = align256(o + 12 * (size_t)G);  // three rotating [G] count buffers
-  l.total = o;
+  l.ctl = o; o = align256(o + sizeof(LvCtl) + 4);  // and the sort's item count
+  l.cnt = o; o = align256(o + 4 * N);
+  l.packed = o; o = align256(o + sizeof(int4) * N);
+  l.spill = o; o = align256(o + 8 * N);
+  l.hist = o; o = align256(o + 4 * (size_t)kDigits * lv_tiles(n).tiles);
+  l.total = o + 16;
   return l;
+}
+
+// The records are read and written as 16-byte vectors.
+char* lv_base(void* ws) { return (char*)(((uintptr_t)ws + 15) & ~(uintptr_t)15); }
+
+template <class... P, class... A>
+cudaError_t lv_launch(void (*kern)(P...), int grid, int block, size_t smem, bool overlap,
+                      cudaStream_t st, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = at;
+  cfg.numAttrs = overlap ? 1 : 0;
+  count_launch();
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 }  // namespace
@@ -813,9 +774,8 @@ extern "C" {
 otg_status otg_levelize_workspace_size(int32_t n, int32_t num_edges, size_t* bytes) {
   (void)num_edges;
   if (!bytes || n < 0) return OTG_ERR_INVALID;
-  otg::LvDev& d = otg::lv_dev();
-  if (d.sms <= 0) return OTG_ERR_CUDA;
-  *bytes = otg::lv_ws(n, d.sms * d.occ).total;
+  if (otg::lv_dev().sms <= 0) return OTG_ERR_CUDA;
+  *bytes = otg::lv_ws(n).total;
   return OTG_OK;
 }
 
@@ -831,65 +791,70 @@ otg_status otg_levelize(int32_t n, int32_t num_edges, const int32_t* fanin_start
                 (num_edges && !fanin)))
     return OTG_ERR_INVALID;
   otg::LvDev& d = otg::lv_dev();
-  int G = d.sms * d.occ;
-  const otg::LvWs l = otg::lv_ws(n, G);
+  const otg::LvWs l = otg::lv_ws(n);
   if (workspace_bytes < l.total) return OTG_ERR_WORKSPACE;
-  const int nw = (n + 31) / 32;
+  char* ws = otg::lv_base(workspace);
+  cudaStream_t st = (cudaStream_t)stream;
+  otg::LvArgs a{n,     fanin_start, fanin,      out_deg, frontier0,
+                first_size, order,  level,      level_ends, counts,
+                (otg::LvCtl*)(ws + l.ctl), (int*)(ws + l.cnt), (int4*)(ws + l.packed),
+                (int*)(ws + l.spill)};
   const otg::ClPlan pl = otg::lv_cluster_plan(n, d);
-  if (pl.S > 0) {
-    char* ws = (char*)workspace;
-    cudaStream_t s = (cudaStream_t)stream;
-    if (cudaMemsetAsync(ws + l.ctl, 0, sizeof(otg::LvCtl), s) != cudaSuccess) return OTG_ERR_CUDA;
-    otg::LvCtl* ctl = (otg::LvCtl*)(ws + l.ctl);
-    int* cnt = (int*)(ws + l.cnt);
-    int cshift = pl.cshift;
-    int lst_cap = otg::lv_lst_cap(1 << pl.cshift, pl.scnt);
-    int scnt_on = pl.scnt ? 1 : 0;
+  const bool on_chip = pl.S > 0 && pl.scnt;
+  cudaError_t e = otg::lv_launch(otg::levelize_pack, std::max(1, std::min((n + 255) / 256, 8 * d.sms)),
+                                 256, 0, false, st, a, !on_chip);
+  if (e == cudaSuccess && first_size > 0) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)pl.S;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(pl.S);
-    cfg.blockDim = dim3(otg::kWidths[pl.wi]);
-    cfg.dynamicSmemBytes = otg::kClusterSmemMax;
-    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    cfg.stream = st;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
-    void* args[] = {&n,          (void*)&fanin_start, (void*)&fanin, (void*)&out_deg,
-                    (void*)&frontier0, &first_size, &order, &level, &level_ends, &counts,
-                    &ctl,        &cnt,        &cshift,       &lst_cap,  &scnt_on};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, otg::cluster_fn(pl.wi), args);
+    if (pl.S > 0) {
+      at[0].id = cudaLaunchAttributeClusterDimension;
+      at[0].val.clusterDim.x = (unsigned)pl.S;
+      at[0].val.clusterDim.y = 1;
+      at[0].val.clusterDim.z = 1;
+      // its counters are filled while the records are packed
+      at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.numAttrs = 2;
+      cfg.gridDim = dim3(pl.S);
+      cfg.blockDim = dim3(otg::kWidths[pl.wi]);
+      cfg.dynamicSmemBytes = otg::kClusterSmemMax;
+      int cap = pl.cap, scnt = on_chip ? 1 : 0;
+      void* args[] = {&a, &cap, &scnt};
+      e = cudaLaunchKernelExC(&cfg, otg::cluster_fn(pl.wi), args);
+    } else {
+      void* args[] = {&a};
+      e = cudaLaunchCooperativeKernel((const void*)otg::levelize_grid_kernel, dim3(d.sms),
+                                      dim3(otg::LT), args, otg::kGridSmem, st);
+    }
     otg::count_launch();
-    return e == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
   }
-  // Small graphs take fewer CTAs: a range of at least kWordsPerCta bitmap
-  // words each, so that fewer CTAs meet at every level's grid barrier.  On a
-  // 165k-pin, 600-level graph, 81 CTAs took 4.16 ms where 296 took 4.50
-  // (6 and 21 CTAs: 4.32 and 4.42); graphs of 5M pins keep every CTA.
-  constexpr int kWordsPerCta = 64;
-  G = std::max(1, std::min(G, (nw + kWordsPerCta - 1) / kWordsPerCta));
-  char* ws = (char*)workspace;
-  cudaStream_t s = (cudaStream_t)stream;
-  if (cudaMemsetAsync(ws + l.ctl, 0, sizeof(otg::LvCtl), s) != cudaSuccess) return OTG_ERR_CUDA;
-  otg::LvCtl* ctl = (otg::LvCtl*)(ws + l.ctl);
-  int* cnt = (int*)(ws + l.cnt);
-  unsigned* bm0 = (unsigned*)(ws + l.bm0);
-  unsigned* bm1 = (unsigned*)(ws + l.bm1);
-  int* blk = (int*)(ws + l.blk);
-  void* args[] = {&n,     (void*)&fanin_start, (void*)&fanin, (void*)&out_deg, (void*)&frontier0,
-                  &first_size, &order, &level, &level_ends, &counts, &ctl, &cnt, &bm0, &bm1, &blk};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)otg::levelize_kernel, dim3(G),
-                                              dim3(otg::LT), args, 0, s);
-  otg::count_launch();
-  return e == cudaSuccess ? OTG_OK : OTG_ERR_CUDA;
+  otg::LvSort s = otg::lv_tiles(n);
+  s.hist = (int*)(ws + l.hist);
+  s.first = (int*)(ws + l.packed);  // the records have been read
+  s.num = (int*)(ws + l.ctl + sizeof(otg::LvCtl));
+  for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {
+    if (pass == 1 && n <= otg::kDigits + 1) break;  // a level has at least one pin
+    e = otg::lv_launch(otg::levelize_hist, s.tiles, otg::ST, 0, pass > 0, st, a, s, pass);
+    if (e == cudaSuccess)
+      e = otg::lv_launch(otg::levelize_scan, 1, otg::kDigits, 0, true, st, a, s, pass);
+    if (e == cudaSuccess)
+      e = otg::lv_launch(otg::levelize_scatter, s.tiles, otg::ST, otg::kScatterSmem, true, st, a, s,
+                         pass);
+    if (e == cudaSuccess && pass == 1)
+      e = otg::lv_launch(otg::levelize_ends, std::max(1, std::min((n + 255) / 256, 4 * d.sms)), 256,
+                         0, true, st, a, s);
+  }
+  if (e == cudaSuccess) return OTG_OK;
+  cudaGetLastError();
+  return OTG_ERR_CUDA;
 }
 
 otg_status otg_levelize_status(const void* workspace, otg_stream_t stream) {
   if (!workspace) return OTG_ERR_INVALID;
-  otg::LvCtl h;
-  if (cudaMemcpyAsync(&h, workspace, sizeof(h), cudaMemcpyDeviceToHost, (cudaStream_t)stream) !=
+  otg::GridCtl h;
+  if (cudaMemcpyAsync(&h, otg::lv_base((void*)workspace), sizeof(h), cudaMemcpyDeviceToHost, (cudaStream_t)stream) !=
           cudaSuccess ||
       cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess)
     return OTG_ERR_CUDA;
