@@ -309,13 +309,9 @@ struct ClusterGroup {
   long long* xch = nullptr;  // this CTA's exchange slot [2] (its own shared memory)
   __device__ int vt() const { return S * T; }
   __device__ int rank() const { return r * T + (int)threadIdx.x; }
-  // The cluster barrier orders the workspace writes of every CTA (release
-  // at arrive, acquire at wait); the fence after it also keeps each SM from
-  // serving a later read of the workspace from a line it cached before.
-  __device__ void sync() const {
-    cg::this_cluster().sync();
-    __threadfence();
-  }
+  // The cluster barrier orders the workspace accesses of every CTA (release
+  // at arrive, acquire at wait).
+  __device__ void sync() const { cg::this_cluster().sync(); }
   // the CTAs' totals of a pair of values: this CTA's exclusive base and the
   // group total (two cluster barriers: publish, then free the slot again)
   __device__ void cta_bases(long long t0, long long t1, long long (&base)[2],
