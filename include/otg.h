@@ -198,7 +198,7 @@ void otg_release_host_context(void);
  * on the GPU race, so serialize them.  Blocks until `stream` finishes and
  * returns the device-side status of the call.  Limit: at most 524,284 nets
  * per call and no net beyond the shared-memory classes of the device's
- * tuning (4,265 nodes on a B200 with the default tuning); larger batches
+ * tuning (4,888 nodes on a B200 with the default tuning); larger batches
  * return OTG_ERR_WORKSPACE without launching.  Allocates nothing.
  */
 otg_status otg_rc_timing_noalloc(const otg_rc_forest* forest, int32_t max_net_nodes,
@@ -305,7 +305,9 @@ typedef struct otg_rc_tuning {
   int32_t class_items[6];
 } otg_rc_tuning;
 otg_status otg_rc_get_tuning(otg_rc_tuning* tuning);
-/* NULL restores the default; OTG_ERR_INVALID for a tuning that does not
+/* NULL restores the default (while nothing is set, a pass of few nets takes a
+ * default with more threads per net; otg_rc_get_tuning returns the one for
+ * many); OTG_ERR_INVALID for a tuning that does not
  * validate (nothing changes). */
 otg_status otg_rc_set_tuning(const otg_rc_tuning* tuning);
 /* Autotuner: times candidate tunings on a sample forest (device pointers;

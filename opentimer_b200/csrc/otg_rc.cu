@@ -979,8 +979,11 @@ __host__ __device__ inline uint32_t rc_smem_bytes(int n, int T, int K, bool tile
 
 // `few`: a class of at most this many items is left to the cluster kernel
 // (the huge-net class; 0 elsewhere).
+// The tile kernel gets 64 registers, so that 1024 threads fit an SM at every
+// size; with 90, and three items' reads in flight at once, a net takes 26%
+// less time and the pass 45% more.
 template <int T, int K, class Ix, bool SMEM, bool TILE = false>
-__global__ void __launch_bounds__(T) rc_block_kernel(RcJob job, const int* list, const int* count,
+__global__ void __launch_bounds__(T, TILE ? 1024 / T : 1) rc_block_kernel(RcJob job, const int* list, const int* count,
                                                      int* work, char* gws, size_t ws_stride,
                                                      int few) {
   extern __shared__ __align__(16) char dsm[];
@@ -1130,6 +1133,17 @@ constexpr Shape kShapeSet[] = {{64, 4},  {64, 8},  {128, 4}, {128, 8}, {256, 2},
                                {256, 8}, {512, 2}, {512, 4}, {512, 8}, {1024, 2}, {1024, 4}};
 constexpr int kNumShapes = (int)(sizeof(kShapeSet) / sizeof(kShapeSet[0]));
 constexpr int kBlockClasses = 6;
+// Largest net of the tile kernel's classes; larger ones go to the huge class
+// (and, when there are few, to clusters).
+constexpr int kTileMax = 4888;
+// With many nets a class of nets up to this size runs one warp per net,
+// whatever its shape: nets of 33..64, 65..128, 129..200 nodes at 4.6, 6.2,
+// 7.4 nodes/ns against 3.0, 4.7, 6.9 with two warps; of 201..310 at 6.6
+// against 8.0.
+constexpr int kWarpTileMax = 200;
+// Nets per SM of a pass up to which the default table gives a net more
+// threads (see default_tune).
+constexpr int kFewNets = 8, kSomeNets = 20;
 
 int shape_index(int T, int K) {
   for (int s = 0; s < kNumShapes; ++s)
@@ -1150,7 +1164,7 @@ bool rc_use_tile() {
 // Largest n whose 16-bit block layout fits the shared-memory budget.
 int rc_smem_nmax(int T, int K, int smem_budget) {
   const bool tile = rc_use_tile();
-  int lo = 33, hi = 32767;
+  int lo = 33, hi = tile ? kTileMax : 32767;
   if (rc_smem_bytes(lo, T, K, tile) > (uint32_t)smem_budget) return 32;
   while (lo < hi) {
     const int mid = (lo + hi + 1) / 2;
@@ -1170,18 +1184,37 @@ struct RcTune {
   int shape[kBlockClasses] = {};
 };
 
-RcTune default_tune(int smem_budget) {
+// The default table for a pass of `nets` nets of at most max_net_nodes.
+// Many nets: the fewest threads that keep an SM's shared memory and warps
+// busy, and narrow classes (a class's shared memory is that of its largest
+// net): 20,000 nets of 2..512 nodes in 307 us, 367 with bounds 200, 420, 900.
+// Few: the pass lasts as long as its largest net, and every class adds a
+// launch, so wide classes with more threads: 500 nets in 47 us against 68,
+// 2,500 nets in 74 against 89 (with the table for few 93; 5,000 nets: 118 and
+// 160 against 100).
+RcTune default_tune(int smem_budget, long long nets, int max_net_nodes, int sms) {
+  struct Row {
+    int nmax;
+    Shape s;
+  };
+  // 2496: the most that leave room for two CTAs of 512 threads on an SM
+  constexpr Row many[] = {{128, {64, 4}},  {256, {64, 8}},   {512, {128, 8}},
+                          {1024, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
+  constexpr Row some[] = {{512, {128, 8}}, {1024, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
+  const Row few[] = {{512, {max_net_nodes <= 128 ? 128 : 256, 4}}, {1024, {512, 4}}, {0, {1024, 4}}};
   RcTune t;
-  const int bounds[kBlockClasses - 1] = {128, 256, 512, 1024, 2048};
-  const Shape shapes[kBlockClasses] = {{64, 4}, {64, 8}, {128, 8}, {256, 4}, {256, 8}, {1024, 4}};
-  t.num = kBlockClasses;
-  for (int c = 0; c < kBlockClasses; ++c) {
-    t.shape[c] = shape_index(shapes[c].T, shapes[c].K);
-    t.nmax[c] = c < kBlockClasses - 1 ? bounds[c] : 0;
-  }
-  t.nmax[kBlockClasses - 1] =
-      std::max(bounds[kBlockClasses - 2] + 1, rc_smem_nmax(shapes[kBlockClasses - 1].T,
-                                                           shapes[kBlockClasses - 1].K, smem_budget));
+  auto fill = [&](const Row* rows, int num) {
+    t.num = num;
+    for (int c = 0; c < num; ++c) {
+      t.shape[c] = shape_index(rows[c].s.T, rows[c].s.K);
+      t.nmax[c] = rows[c].nmax;
+    }
+    t.nmax[num - 1] = std::max(t.nmax[num - 2] + 1,
+                               rc_smem_nmax(rows[num - 1].s.T, rows[num - 1].s.K, smem_budget));
+  };
+  if (nets > (long long)kSomeNets * sms) fill(many, 6);
+  else if (nets > (long long)kFewNets * sms) fill(some, 4);
+  else fill(few, 3);
   return t;
 }
 
@@ -1191,6 +1224,7 @@ bool tune_ok(const RcTune& t, int smem_budget) {
   for (int c = 0; c < t.num; ++c) {
     if (t.shape[c] < 0 || t.shape[c] >= kNumShapes || t.nmax[c] <= prev) return false;
     const Shape sh = kShapeSet[t.shape[c]];
+    if (rc_use_tile() && t.nmax[c] > kTileMax) return false;
     if (rc_smem_bytes(t.nmax[c], sh.T, sh.K, rc_use_tile()) > (uint32_t)smem_budget) return false;
     prev = t.nmax[c];
   }
@@ -1212,15 +1246,22 @@ std::mutex g_tune_mu;
 RcTune g_tune[64];
 bool g_tune_set[64] = {};
 
-RcTune current_tune(int smem_budget) {
+// The tuning that was set, else the default for such a pass.
+RcTune current_tune(int smem_budget, long long nets, int max_net_nodes, int sms) {
+  int d = 0;
+  cudaGetDevice(&d);
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    if (g_tune_set[d & 63]) return g_tune[d & 63];
+  }
+  return default_tune(smem_budget, nets, max_net_nodes, sms);
+}
+
+void clear_tune() {
   int d = 0;
   cudaGetDevice(&d);
   std::lock_guard<std::mutex> lk(g_tune_mu);
-  if (!g_tune_set[d & 63]) {
-    g_tune[d & 63] = default_tune(smem_budget);
-    g_tune_set[d & 63] = true;
-  }
-  return g_tune[d & 63];
+  g_tune_set[d & 63] = false;
 }
 
 void set_tune(const RcTune& t) {
@@ -1330,7 +1371,8 @@ size_t rc_workspace_bytes_for(const RcTune& t, int num_nets, int max_net_nodes, 
 
 size_t rc_workspace_bytes(int num_nets, int max_net_nodes, int sms, int smem_budget,
                           size_t* off_lists, size_t* off_huge, size_t* huge_stride) {
-  return rc_workspace_bytes_for(current_tune(smem_budget), num_nets, max_net_nodes, sms,
+  return rc_workspace_bytes_for(current_tune(smem_budget, num_nets, max_net_nodes, sms), num_nets,
+                                max_net_nodes, sms,
                                 off_lists, off_huge, huge_stride);
 }
 
@@ -1364,9 +1406,14 @@ cudaError_t chain_launch(void (*kern)(P...), int grid, int block, size_t smem, i
 
 template <int T, int K>
 cudaError_t launch_smem_class(const RcJob& job, const int* list, int* count, int* work, int nmax,
-                              int sms, bool chained, cudaStream_t stream) {
+                              int sms, bool many, bool chained, cudaStream_t stream) {
   const bool tile = rc_use_tile();
-  auto kern = tile ? rc_block_kernel<T, K, uint16_t, true, true> : rc_block_kernel<T, K, uint16_t, true>;
+  if constexpr (T > 32)
+    if (tile && many && nmax <= kWarpTileMax)
+      return launch_smem_class<32, 4>(job, list, count, work, nmax, sms, many, chained, stream);
+  auto kern = rc_block_kernel<T, K, uint16_t, true, true>;
+  if constexpr (T > 32)
+    if (!tile) kern = rc_block_kernel<T, K, uint16_t, true>;
   const size_t smem = rc_smem_bytes(nmax, T, K, tile);
   // The attribute is always set to the same (largest) value, so threads
   // launching with different nmax never lower it under one another.
@@ -1381,20 +1428,20 @@ cudaError_t launch_smem_class(const RcJob& job, const int* list, int* count, int
 }
 
 cudaError_t launch_shape(int s, const RcJob& job, const int* list, int* count, int* work,
-                         int nmax, int sms, bool chained, cudaStream_t st) {
+                         int nmax, int sms, bool many, bool chained, cudaStream_t st) {
   switch (s) {
-    case 0: return launch_smem_class<64, 4>(job, list, count, work, nmax, sms, chained, st);
-    case 1: return launch_smem_class<64, 8>(job, list, count, work, nmax, sms, chained, st);
-    case 2: return launch_smem_class<128, 4>(job, list, count, work, nmax, sms, chained, st);
-    case 3: return launch_smem_class<128, 8>(job, list, count, work, nmax, sms, chained, st);
-    case 4: return launch_smem_class<256, 2>(job, list, count, work, nmax, sms, chained, st);
-    case 5: return launch_smem_class<256, 4>(job, list, count, work, nmax, sms, chained, st);
-    case 6: return launch_smem_class<256, 8>(job, list, count, work, nmax, sms, chained, st);
-    case 7: return launch_smem_class<512, 2>(job, list, count, work, nmax, sms, chained, st);
-    case 8: return launch_smem_class<512, 4>(job, list, count, work, nmax, sms, chained, st);
-    case 9: return launch_smem_class<512, 8>(job, list, count, work, nmax, sms, chained, st);
-    case 10: return launch_smem_class<1024, 2>(job, list, count, work, nmax, sms, chained, st);
-    case 11: return launch_smem_class<1024, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 0: return launch_smem_class<64, 4>(job, list, count, work, nmax, sms, many, chained, st);
+    case 1: return launch_smem_class<64, 8>(job, list, count, work, nmax, sms, many, chained, st);
+    case 2: return launch_smem_class<128, 4>(job, list, count, work, nmax, sms, many, chained, st);
+    case 3: return launch_smem_class<128, 8>(job, list, count, work, nmax, sms, many, chained, st);
+    case 4: return launch_smem_class<256, 2>(job, list, count, work, nmax, sms, many, chained, st);
+    case 5: return launch_smem_class<256, 4>(job, list, count, work, nmax, sms, many, chained, st);
+    case 6: return launch_smem_class<256, 8>(job, list, count, work, nmax, sms, many, chained, st);
+    case 7: return launch_smem_class<512, 2>(job, list, count, work, nmax, sms, many, chained, st);
+    case 8: return launch_smem_class<512, 4>(job, list, count, work, nmax, sms, many, chained, st);
+    case 9: return launch_smem_class<512, 8>(job, list, count, work, nmax, sms, many, chained, st);
+    case 10: return launch_smem_class<1024, 2>(job, list, count, work, nmax, sms, many, chained, st);
+    case 11: return launch_smem_class<1024, 4>(job, list, count, work, nmax, sms, many, chained, st);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1449,7 +1496,7 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
   if (!workspace || cap < 0 || max_net_nodes < 1) return OTG_ERR_INVALID;
   DevInfo& di = dev_info();
   const int budget = di.smem_optin - kStaticSmemReserve;
-  const RcTune tn = tune ? *tune : current_tune(budget);
+  const RcTune tn = tune ? *tune : current_tune(budget, cap, max_net_nodes, di.sms);
   size_t off_lists, off_huge, stride;
   const size_t need = rc_workspace_bytes_for(tn, std::max(cap, 1), max_net_nodes, di.sms,
                                              &off_lists, &off_huge, &stride);
@@ -1512,8 +1559,8 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
     if (max_net_nodes <= cls.nmax[c - 1]) continue;
     const int nmax = std::min(cls.nmax[c], max_net_nodes);
     cudaStream_t st = next_stream();
-    err = launch_shape(tn.shape[c - 1], job, L(c), counters + c, work + c, nmax, di.sms, chained,
-                       st);
+    err = launch_shape(tn.shape[c - 1], job, L(c), counters + c, work + c, nmax, di.sms,
+                       cap > kSomeNets * (long long)di.sms, chained, st);
   }
   if (err == cudaSuccess) {
     cudaStream_t st = next_stream();
@@ -1624,7 +1671,7 @@ otg_status rc_autotune(const otg_rc_forest* f, int max_net_nodes, cudaStream_t s
     }
     return best;
   };
-  RcTune best = current_tune(budget);
+  RcTune best = current_tune(budget, f->num_nets, max_net_nodes, di.sms);
   float tb = time_of(best);
   auto consider = [&](const RcTune& t) {
     if (err != OTG_OK || !tune_ok(t, budget)) return;
@@ -1733,7 +1780,9 @@ otg_status otg_rc_get_tuning(otg_rc_tuning* out) {
   if (!out) return OTG_ERR_INVALID;
   otg::DevInfo& di = otg::dev_info();
   if (di.sms <= 0) return OTG_ERR_CUDA;
-  otg::to_c(otg::current_tune(di.smem_optin - otg::kStaticSmemReserve), out);
+  // without a tuning set: the default for many nets
+  otg::to_c(otg::current_tune(di.smem_optin - otg::kStaticSmemReserve, 1ll << 40, 1 << 30, di.sms),
+            out);
   return OTG_OK;
 }
 
@@ -1741,8 +1790,12 @@ otg_status otg_rc_set_tuning(const otg_rc_tuning* t) {
   otg::DevInfo& di = otg::dev_info();
   if (di.sms <= 0) return OTG_ERR_CUDA;
   const int budget = di.smem_optin - otg::kStaticSmemReserve;
-  otg::RcTune tn = otg::default_tune(budget);
-  if (t && (!otg::from_c(t, &tn) || !otg::tune_ok(tn, budget))) return OTG_ERR_INVALID;
+  if (!t) {
+    otg::clear_tune();
+    return OTG_OK;
+  }
+  otg::RcTune tn;
+  if (!otg::from_c(t, &tn) || !otg::tune_ok(tn, budget)) return OTG_ERR_INVALID;
   otg::set_tune(tn);
   return OTG_OK;
 }

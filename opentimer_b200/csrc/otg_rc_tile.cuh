@@ -24,11 +24,17 @@
 //   T7  BFS slots: stable radix sort by depth of the ids in descending
 //       order, the reference's (distance asc, local id desc) rule
 //       (sort.cuh:102-121); node2bfs, pid.
-// Elmore (E1-E9), one corner pair at a time, with exact int64 fixed-point
-// sums (fx_scale): load and ldelay are subtree sums, taken as differences
-// of an exclusive prefix over the preorder; delay and beta are path sums,
-// taken as a prefix over the signed Euler tour of per-node int64 terms
-// that are converted once per node, so the tour scans only add integers.
+// Elmore, one corner pair at a time, with exact int64 fixed-point sums
+// (fx_scale): load and ldelay are subtree sums, taken as differences of an
+// exclusive prefix over the preorder; delay and beta are path sums, taken as
+// the prefix over the preorder less the prefix over the postorder of the
+// nodes left before (a node's term goes straight to its postorder place
+// i - depth + size - 1).  That is two prefixes of n terms read in order,
+// where a signed prefix over the Euler tour gathers 2(n-1) terms by index
+// twice over (2049..4096 nodes: 6.25 -> 6.65 nodes/ns, 81 -> 77 warp
+// instructions and 28.8 -> 26 shared-memory wavefronts per node).  What
+// bounds the kernel is the load/store unit, 61% busy over all phases and
+// barriers; HBM is at 12%.
 // Every scan is one tile: thread t owns an odd number KE of consecutive
 // items (odd, so strided 8- and 16-byte accesses spread over the banks),
 // sums them, and the block-wide base comes from the warp totals after a
@@ -37,7 +43,7 @@
 // ---- layout -------------------------------------------------------------
 struct RcTileLayout {
   // persistent
-  uint32_t pre, psz, bpre, code, pres;
+  uint32_t pre, bpre, nd;
   // topology scratch (T1-T7)
   uint32_t E, PX, deg, off, succ, sidx, subrk, spos, sl, db, dbp, depth, par, slot, rbuf, hist;
   // Elmore (E1-E9), overlaying the topology scratch
@@ -58,10 +64,8 @@ __host__ __device__ inline RcTileLayout rc_tile_layout(int n, int T) {
     o = OTG_AL(o + (bytes)); \
   } while (0)
   OTG_TAKE(pre, 2u * N);
-  OTG_TAKE(psz, 2u * N);
   OTG_TAKE(bpre, 2u * N);
-  OTG_TAKE(code, 2u * A);
-  OTG_TAKE(pres, 4u * N);
+  OTG_TAKE(nd, 8u * N);
   const uint32_t scratch = o;
   // topology
   OTG_TAKE(E, 4u * M);
@@ -126,70 +130,43 @@ __device__ __forceinline__ int tile_excl_i32(int v, int* wt, int* total) {
   return before + x - v;
 }
 
-__device__ __forceinline__ long long shfl_up_ll(long long v, int d) {
-  return __shfl_up_sync(FULL, v, d);
-}
+// Sum over the warp's lanes (mod 2^64), as three 32-bit reductions of 22,
+// 22 and 20 bits a lane.
 __device__ __forceinline__ long long warp_sum_ll(long long v) {
-#pragma unroll
-  for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(FULL, v, d);
-  return v;
+  const unsigned long long x = (unsigned long long)v;
+  const unsigned lo = __reduce_add_sync(FULL, (unsigned)x & 0x3FFFFFu);
+  const unsigned mid = __reduce_add_sync(FULL, (unsigned)(x >> 22) & 0x3FFFFFu);
+  const unsigned hi = __reduce_add_sync(FULL, (unsigned)(x >> 44));
+  return (long long)(lo + ((unsigned long long)mid << 22) + ((unsigned long long)hi << 44));
 }
 
-// Exclusive block base of a pair of int64 values (one pair per thread),
-// one barrier.  wt holds 2*(T/32) int64.
-template <int T>
-__device__ __forceinline__ void tile_excl_i64x2(long long a0, long long a1, long long* wt,
-                                                long long& e0, long long& e1) {
+// Exclusive block base of N int64 values per thread (in: the thread's sums,
+// out: the sums of the threads before it), one barrier.  wt holds N*(T/32)
+// int64; the caller has a barrier between two uses of it.
+template <int T, int N>
+__device__ __forceinline__ void tile_excl_i64(long long (&v)[N], long long* wt) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int W = T / 32;
-  long long x0 = a0, x1 = a1;
+  long long x[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) x[j] = v[j];
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const long long y0 = shfl_up_ll(x0, d), y1 = shfl_up_ll(x1, d);
-    if (lane >= d) {
-      x0 += y0;
-      x1 += y1;
-    }
+    long long y[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) y[j] = __shfl_up_sync(FULL, x[j], d);
+#pragma unroll
+    for (int j = 0; j < N; ++j) x[j] += lane >= d ? y[j] : 0;
   }
   if (lane == 31) {
-    wt[2 * w] = x0;
-    wt[2 * w + 1] = x1;
+#pragma unroll
+    for (int j = 0; j < N; ++j) wt[N * w + j] = x[j];
   }
   __syncthreads();
-  long long b0 = 0, b1 = 0;
-  if (lane < w && lane < W) {
-    b0 = wt[2 * lane];
-    b1 = wt[2 * lane + 1];
-  }
-  e0 = warp_sum_ll(b0) + x0 - a0;
-  e1 = warp_sum_ll(b1) + x1 - a1;
-}
-
-// Exclusive fixed-point scan of a corner pair over C items: term(i) gives
-// item i's two int64 terms, emit(i, e0, e1, t) receives the exclusive
-// prefix before item i and the item's terms.  Thread t owns items
-// [t*KE, t*KE+KE); the terms are evaluated twice (sum, then emit), which
-// keeps no per-item state in registers.
-template <int T, class TermF, class EmitF>
-__device__ __forceinline__ void scan_pair(int C, TermF term, EmitF emit, long long* wt) {
-  const int KE = tile_items(C, T);
-  const int i0 = threadIdx.x * KE;
-  const int i1 = min(i0 + KE, C);
-  long long s0 = 0, s1 = 0;
-#pragma unroll 3
-  for (int i = i0; i < i1; ++i) {
-    const longlong2 t = term(i);
-    s0 += t.x;
-    s1 += t.y;
-  }
-  long long e0, e1;
-  tile_excl_i64x2<T>(s0, s1, wt, e0, e1);
-#pragma unroll 3
-  for (int i = i0; i < i1; ++i) {
-    const longlong2 t = term(i);
-    emit(i, e0, e1, t);
-    e0 += t.x;
-    e1 += t.y;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const long long before = lane < w && lane < W ? wt[N * lane + j] : 0;
+    v[j] = warp_sum_ll(before) + x[j] - v[j];
   }
 }
 
@@ -204,6 +181,10 @@ __device__ __forceinline__ void commit_max(float m, unsigned* dst) {
   if ((threadIdx.x & 31) == 0 && x) atomicMax(dst, x);
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
 // ---- the net --------------------------------------------------------------
 template <int T>
 __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, long long* shl) {
@@ -216,10 +197,8 @@ __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, 
   const int m = n - 1, A = 2 * m, eb = b - net;
   const RcTileLayout L = rc_tile_layout(n, T);
   Ix* pre = (Ix*)(ws + L.pre);
-  Ix* psz = (Ix*)(ws + L.psz);
   Ix* bpre = (Ix*)(ws + L.bpre);
-  int16_t* code = (int16_t*)(ws + L.code);
-  float* pres = (float*)(ws + L.pres);
+  uint2* nd = (uint2*)(ws + L.nd);  // by preorder: depth | subtree size << 16, parent resistance
   unsigned* E = (unsigned*)(ws + L.E);
   unsigned* PX = (unsigned*)(ws + L.PX);
   unsigned* deg = (unsigned*)(ws + L.deg);
@@ -271,6 +250,13 @@ __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, 
   if (tid < 16) smx[tid] = 0u;
   const int NW = (n + 1) >> 1;
   for (int w = tid; w < NW; w += T) deg[w] = 0u;
+  // The caps and resistances, read many phases later, into L2: with one or
+  // two CTAs on the SM nothing else hides their latency (2049..4096 nodes:
+  // 6.65 -> 6.8 nodes/ns; smaller nets: no gain).
+  if constexpr (T >= 512) {
+    for (int v = 8 * tid; v < n; v += 8 * T) prefetch_l2(a.cap + b + v);
+    for (int e = 32 * tid; e < m; e += 32 * T) prefetch_l2(g_res + eb + e);
+  }
   __syncthreads();
   for (int e = tid; e < m; e += T) {
     int2 ed = g_edges[eb + e];
@@ -434,8 +420,7 @@ __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, 
   }
   if (tid == 0) {
     pre[root] = 0;
-    psz[0] = (Ix)n;
-    pres[0] = 0.0f;
+    nd[0] = make_uint2((unsigned)n << 16, 0u);
     depth[root] = 0;
     par[root] = (Ix)root;
   }
@@ -452,10 +437,8 @@ __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, 
       pre[ch] = (Ix)pv;
       depth[ch] = (Ix)d;
       par[ch] = (Ix)(pc & 0xFFFFu);
-      psz[pv] = (Ix)((ex - en + 1) >> 1);
-      pres[pv] = g_res[eb + e];
-      code[en] = (int16_t)(pv + 1);
-      code[ex] = (int16_t)(-(pv + 1));
+      nd[pv] = make_uint2((unsigned)d | (unsigned)((ex - en + 1) >> 1) << 16,
+                          __float_as_uint(g_res[eb + e]));
       dmax = max(dmax, d);
     }
     dmax = __reduce_max_sync(FULL, dmax);
@@ -524,17 +507,28 @@ __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, 
 
   PHASE(8);
   // ---- E: Elmore per corner pair
+  const int KE = tile_items(n, T);
+  const int i0 = tid * KE, i1 = min(i0 + KE, n);
+  // f(i) over this thread's items.  One at a time: reading a few items ahead
+  // takes 90 registers, and what counts is the number of resident warps.
+  auto own = [&](auto f) {
+    for (int i = i0; i < i1; ++i) f(i);
+  };
+  auto res_of = [](uint2 q) { return __uint_as_float(q.y); };
   for (int cp = 0; cp < 2; ++cp) {
-    long long* wtl0 = shl;
-    long long* wtl1 = shl + 2 * W;
-    if (tid < 4) smx[4 + tid] = 0u;  // the pair's sweep maxima (w, delay, w2)
+    // out[slot] = Y[node]: the pair's half of an output, BFS order
+    auto rows_out = [&](float4* rows) {
+      float2* out = (float2*)rows;
+      for (int r = tid; r < n; r += T) out[2 * (size_t)(b + r) + cp] = Y[bpre[r]];
+    };
+    if (tid < 6) smx[4 + tid] = 0u;  // the pair's sweep maxima (w, delay, w2)
     // E0: the pair's caps, read once in id order (coalesced), staged by
-    // preorder in Y (free until the delay sweep), and their maxima
+    // preorder in X, and their maxima
     {
       float m0 = 0.f, m1 = 0.f;
       for (int v = tid; v < n; v += T) {
         const float2 c = cap2[2 * (size_t)(b + v) + cp];
-        Y[pre[v]] = c;
+        X[pre[v]] = c;
         m0 = fmaxf(m0, fabsf(c.x));
         m1 = fmaxf(m1, fabsf(c.y));
       }
@@ -542,190 +536,142 @@ __device__ void rc_net_tile(const RcArgs& a, int net, char* ws, int n, int* sh, 
       commit_max(m1, smx + 2 * cp + 1);
     }
     __syncthreads();
-    float upc[2], dnc[2];
-    fx_scale(__uint_as_float(smx[2 * cp]), n, upc[0], dnc[0]);
-    fx_scale(__uint_as_float(smx[2 * cp + 1]), n, upc[1], dnc[1]);
-    // E1: load scan over the preorder: Ip[i] = exclusive prefix of cap
-    scan_pair<T>(
-        n,
-        [&](int i) {
-          const float2 c = Y[i];
-          return make_longlong2(to_fx(c.x, upc[0]), to_fx(c.y, upc[1]));
-        },
-        [&](int i, long long e0, long long e1, longlong2 t) {
-          Ip[i] = make_longlong2(e0, e1);
-          if (i == n - 1) Ip[n] = make_longlong2(e0 + t.x, e1 + t.y);  // the total
-        },
-        wtl0);
-    __syncthreads();
+    // Ip[i] = exclusive prefix over the preorder of fx(term(i)); Ip[n] = total
+    auto pre_scan = [&](auto term, const float (&up)[2], auto after) {
+      long long e[2] = {0, 0};
+      own([&](int i) {
+        const float2 t = term(i);
+        e[0] += to_fx(t.x, up[0]);
+        e[1] += to_fx(t.y, up[1]);
+      });
+      tile_excl_i64<T, 2>(e, shl);
+      own([&](int i) {
+        const float2 t = term(i);
+        Ip[i] = make_longlong2(e[0], e[1]);
+        e[0] += to_fx(t.x, up[0]);
+        e[1] += to_fx(t.y, up[1]);
+        if (i == n - 1) Ip[n] = make_longlong2(e[0], e[1]);
+        after(i);
+      });
+      __syncthreads();
+    };
+    // Y[i] = subtree sum, the prefix's difference over the subtree's range;
+    // mx: the maxima of |R * sum|
+    auto subtree = [&](const float (&dn)[2], unsigned* mx) {
+      float m0 = 0.f, m1 = 0.f;
+      own([&](int i) {
+        const uint2 q = nd[i];
+        const longlong2 lo = Ip[i], hi = Ip[i + (int)(q.x >> 16)];
+        const float2 v = make_float2(from_fx(hi.x - lo.x, dn[0]), from_fx(hi.y - lo.y, dn[1]));
+        Y[i] = v;
+        m0 = fmaxf(m0, fabsf(v.x * res_of(q)));
+        m1 = fmaxf(m1, fabsf(v.y * res_of(q)));
+      });
+      commit_max(m0, mx);
+      commit_max(m1, mx + 1);
+      __syncthreads();
+    };
+    // emit(i, s0, s1): the path sum of fx(R * Y) from the root to node i, the
+    // prefix over the preorder less that over the nodes left before i is
+    // entered (postorder; i - depth of them).  Y goes out to rows on the way.
+    auto path = [&](const float (&up)[2], float4* rows, auto emit) {
+      auto term = [&](int i, uint2 q) {
+        const float2 v = Y[i];
+        const float r = res_of(q);
+        return i == 0 ? make_longlong2(0, 0)
+                      : make_longlong2(to_fx(v.x * r, up[0]), to_fx(v.y * r, up[1]));
+      };
+      long long e[4] = {0, 0, 0, 0};
+      own([&](int i) {
+        const uint2 q = nd[i];
+        const longlong2 w = term(i, q);
+        e[0] += w.x;
+        e[1] += w.y;
+        // the node's place in the postorder
+        Ip[i - (int)(q.x & 0xFFFFu) + (int)(q.x >> 16) - 1] = w;
+      });
+      rows_out(rows);
+      __syncthreads();
+      own([&](int i) {
+        const longlong2 w = Ip[i];
+        e[2] += w.x;
+        e[3] += w.y;
+      });
+      tile_excl_i64<T, 4>(e, shl);
+      own([&](int i) {
+        const longlong2 w = Ip[i];
+        Ip[i] = make_longlong2(e[2], e[3]);
+        e[2] += w.x;
+        e[3] += w.y;
+      });
+      __syncthreads();
+      own([&](int i) {
+        const uint2 q = nd[i];
+        const longlong2 left = Ip[i - (int)(q.x & 0xFFFFu)], w = term(i, q);
+        e[0] += w.x;
+        e[1] += w.y;
+        emit(i, e[0] - left.x, e[1] - left.y);
+      });
+    };
+    float up[2], dn[2];
+    // load
+    fx_scale(__uint_as_float(smx[2 * cp]), n, up[0], dn[0]);
+    fx_scale(__uint_as_float(smx[2 * cp + 1]), n, up[1], dn[1]);
+    pre_scan([&](int i) { return X[i]; }, up, [](int) {});
     PHASE(10);
-    // E2: load = prefix difference over the subtree's preorder range
-    {
-      const int KE = tile_items(n, T);
-      const int i0 = tid * KE, i1 = min(i0 + KE, n);
-      float mw0 = 0.f, mw1 = 0.f;
-      for (int i = i0; i < i1; ++i) {
-        const longlong2 lo = Ip[i], hi = Ip[i + (int)psz[i]];
-        const float2 v = make_float2(from_fx(hi.x - lo.x, dnc[0]), from_fx(hi.y - lo.y, dnc[1]));
-        X[i] = v;
-        const float r = pres[i];
-        mw0 = fmaxf(mw0, fabsf(v.x * r));
-        mw1 = fmaxf(mw1, fabsf(v.y * r));
-      }
-      commit_max(mw0, smx + 4);
-      commit_max(mw1, smx + 5);
-    }
-    __syncthreads();
+    subtree(dn, smx + 4);
     PHASE(11);
-    // E3: delay terms W = fx(R * load) into Ip; load out in BFS order
-    float upw[2], dnw[2];
-    fx_scale(__uint_as_float(smx[4]), n, upw[0], dnw[0]);
-    fx_scale(__uint_as_float(smx[5]), n, upw[1], dnw[1]);
+    // delay
+    fx_scale(__uint_as_float(smx[4]), n, up[0], dn[0]);
+    fx_scale(__uint_as_float(smx[5]), n, up[1], dn[1]);
     {
-      const int KE = tile_items(n, T);
-      const int i0 = tid * KE, i1 = min(i0 + KE, n);
-      for (int i = i0; i < i1; ++i) {
-        const float2 v = X[i];
-        const float r = pres[i];
-        Ip[i] = make_longlong2(to_fx(v.x * r, upw[0]), to_fx(v.y * r, upw[1]));
-      }
-      float2* out = (float2*)a.load;
-      for (int r = tid; r < n; r += T) out[2 * (size_t)(b + r) + cp] = X[bpre[r]];
-    }
-    if (tid < 2) smx[6 + tid] = 0u;
-    __syncthreads();
-    PHASE(12);
-    // E4: delay = prefix over the signed tour of W; emitted at down arcs.
-    // First the caps move from Y to X (free since the load went out); the
-    // scan's barrier lies between this copy and the first delay written to Y.
-    {
-      const int KE = tile_items(n, T);
-      const int i0 = tid * KE, i1 = min(i0 + KE, n);
-      for (int i = i0; i < i1; ++i) X[i] = Y[i];
-    }
-    {
-      float md0 = 0.f, md1 = 0.f;
-      scan_pair<T>(
-          A,
-          [&](int p) {
-            const int c = (int)code[p];
-            const longlong2 w = Ip[(c > 0 ? c : -c) - 1];
-            return c > 0 ? w : make_longlong2(-w.x, -w.y);
-          },
-          [&](int p, long long e0, long long e1, longlong2 t) {
-            const int c = (int)code[p];
-            if (c > 0) {
-              const float2 d = make_float2(from_fx(e0 + t.x, dnw[0]), from_fx(e1 + t.y, dnw[1]));
-              Y[c - 1] = d;
-              md0 = fmaxf(md0, fabsf(d.x));
-              md1 = fmaxf(md1, fabsf(d.y));
-            }
-          },
-          wtl1);
-      commit_max(md0, smx + 6);
-      commit_max(md1, smx + 7);
-      if (tid == 0) Y[0] = make_float2(0.f, 0.f);
+      float m0 = 0.f, m1 = 0.f;
+      path(up, a.load, [&](int i, long long s0, long long s1) {
+        const float2 d = make_float2(from_fx(s0, dn[0]), from_fx(s1, dn[1]));
+        Y[i] = d;
+        m0 = fmaxf(m0, fabsf(d.x));
+        m1 = fmaxf(m1, fabsf(d.y));
+      });
+      commit_max(m0, smx + 6);
+      commit_max(m1, smx + 7);
     }
     __syncthreads();
     PHASE(13);
-    // E5: ldelay scan over the preorder of cap * delay (scale from the
-    // bound max|cap| * max|delay|); delay out in BFS order
-    float upd[2], dnd[2];
-    fx_scale(__uint_as_float(smx[2 * cp]) * __uint_as_float(smx[6]), n, upd[0], dnd[0]);
-    fx_scale(__uint_as_float(smx[2 * cp + 1]) * __uint_as_float(smx[7]), n, upd[1], dnd[1]);
-    {
-      float2* out = (float2*)a.delay;
-      for (int r = tid; r < n; r += T) out[2 * (size_t)(b + r) + cp] = Y[bpre[r]];
-    }
-    scan_pair<T>(
-        n,
-        [&](int i) {
-          const float2 c = X[i];
-          const float2 d = Y[i];
-          return make_longlong2(to_fx(c.x * d.x, upd[0]), to_fx(c.y * d.y, upd[1]));
-        },
-        [&](int i, long long e0, long long e1, longlong2 t) {
-          Ip[i] = make_longlong2(e0, e1);
-          if (i == n - 1) Ip[n] = make_longlong2(e0 + t.x, e1 + t.y);
-        },
-        wtl0);
-    if (tid < 2) smx[8 + tid] = 0u;
-    __syncthreads();
+    // ldelay (scale from the bound max|cap| * max|delay|); the delay moves to
+    // X behind the cap's last use
+    fx_scale(__uint_as_float(smx[2 * cp]) * __uint_as_float(smx[6]), n, up[0], dn[0]);
+    fx_scale(__uint_as_float(smx[2 * cp + 1]) * __uint_as_float(smx[7]), n, up[1], dn[1]);
+    rows_out(a.delay);
+    pre_scan([&](int i) { return make_float2(X[i].x * Y[i].x, X[i].y * Y[i].y); }, up,
+             [&](int i) { X[i] = Y[i]; });
     PHASE(14);
-    // E6: ldelay = prefix difference over the subtree range
-    {
-      const int KE = tile_items(n, T);
-      const int i0 = tid * KE, i1 = min(i0 + KE, n);
-      float mw0 = 0.f, mw1 = 0.f;
-      for (int i = i0; i < i1; ++i) {
-        const longlong2 lo = Ip[i], hi = Ip[i + (int)psz[i]];
-        const float2 v = make_float2(from_fx(hi.x - lo.x, dnd[0]), from_fx(hi.y - lo.y, dnd[1]));
-        X[i] = v;
-        const float r = pres[i];
-        mw0 = fmaxf(mw0, fabsf(v.x * r));
-        mw1 = fmaxf(mw1, fabsf(v.y * r));
-      }
-      commit_max(mw0, smx + 8);
-      commit_max(mw1, smx + 9);
-    }
-    __syncthreads();
+    subtree(dn, smx + 8);
     PHASE(15);
-    // E7: beta terms into Ip; ldelay out
-    fx_scale(__uint_as_float(smx[8]), n, upw[0], dnw[0]);
-    fx_scale(__uint_as_float(smx[9]), n, upw[1], dnw[1]);
-    {
-      const int KE = tile_items(n, T);
-      const int i0 = tid * KE, i1 = min(i0 + KE, n);
-      for (int i = i0; i < i1; ++i) {
-        const float2 v = X[i];
-        const float r = pres[i];
-        Ip[i] = make_longlong2(to_fx(v.x * r, upw[0]), to_fx(v.y * r, upw[1]));
-      }
-      float2* out = (float2*)a.ldelay;
-      for (int r = tid; r < n; r += T) out[2 * (size_t)(b + r) + cp] = X[bpre[r]];
-    }
-    __syncthreads();
-    PHASE(16);
-    // E8: beta over the signed tour -> impulse = 2 beta - delay^2 (into X)
-    scan_pair<T>(
-        A,
-        [&](int p) {
-          const int c = (int)code[p];
-          const longlong2 w = Ip[(c > 0 ? c : -c) - 1];
-          return c > 0 ? w : make_longlong2(-w.x, -w.y);
-        },
-        [&](int p, long long e0, long long e1, longlong2 t) {
-          const int c = (int)code[p];
-          if (c > 0) {
-            const float2 d = Y[c - 1];
-            X[c - 1] = make_float2(fmaf(-d.x, d.x, 2.0f * from_fx(e0 + t.x, dnw[0])),
-                                   fmaf(-d.y, d.y, 2.0f * from_fx(e1 + t.y, dnw[1])));
-          }
-        },
-        wtl1);
-    if (tid == 0) X[0] = make_float2(0.f, 0.f);
+    // beta -> impulse = 2 beta - delay^2
+    fx_scale(__uint_as_float(smx[8]), n, up[0], dn[0]);
+    fx_scale(__uint_as_float(smx[9]), n, up[1], dn[1]);
+    path(up, a.ldelay, [&](int i, long long s0, long long s1) {
+      const float2 d = X[i];
+      Y[i] = make_float2(fmaf(-d.x, d.x, 2.0f * from_fx(s0, dn[0])),
+                         fmaf(-d.y, d.y, 2.0f * from_fx(s1, dn[1])));
+    });
     __syncthreads();
     PHASE(17);
-    // E9: impulse out; sink slews
-    {
-      float2* out = (float2*)a.impulse;
-      for (int r = tid; r < n; r += T) out[2 * (size_t)(b + r) + cp] = X[bpre[r]];
-      if (a.sinks_start) {
-        const int s0 = a.sinks_start[net], s1 = a.sinks_start[net + 1];
-        const float2 si = ((const float2*)a.driver_slew)[2 * (size_t)net + cp];
-        float2* so = (float2*)a.sink_slew;
-        for (int k = s0 + tid; k < s1; k += T) {
-          const int v = a.sink_nodes[k];
-          if ((unsigned)v >= (unsigned)n) {
-            report(a, OTG_ERR_INVALID, net);
-            continue;
-          }
-          const float2 iv = X[pre[v]];
-          so[2 * (size_t)k + cp] = make_float2(sink_slew1(si.x, iv.x), sink_slew1(si.y, iv.y));
+    rows_out(a.impulse);
+    if (a.sinks_start) {
+      const int s0 = a.sinks_start[net], s1 = a.sinks_start[net + 1];
+      const float2 si = ((const float2*)a.driver_slew)[2 * (size_t)net + cp];
+      float2* so = (float2*)a.sink_slew;
+      for (int k = s0 + tid; k < s1; k += T) {
+        const int v = a.sink_nodes[k];
+        if ((unsigned)v >= (unsigned)n) {
+          report(a, OTG_ERR_INVALID, net);
+          continue;
         }
+        const float2 iv = Y[pre[v]];
+        so[2 * (size_t)k + cp] = make_float2(sink_slew1(si.x, iv.x), sink_slew1(si.y, iv.y));
       }
     }
-    __syncthreads();
     PHASE(18);
   }
 }
