@@ -156,103 +156,117 @@ __device__ __noinline__ float timing_value(const LutSrc& src, const Lut& m, floa
   return m.var == 0 ? lut_eval(m, lutd, a, b) : lut_eval(m, lutd, b, a);
 }
 
-// A cell arc's table at a load that is known before the slew: reduced,
-// while the slew's pin is waited for, to its values along the slew axis at
-// that load, kept in shared memory; what is left for after the wait is the
-// slew's segment (by counting, all axis entries in flight at once) and one
-// interpolation.  In exact arithmetic the same bilinear form as lut_eval's,
-// whichever axis comes first.  Slew axes of up to kPrepAxis entries; others
-// go through timing_value.  After the wait an arc's two tables take about
-// 250 cycles of every gate on a path; interpolating both axes there took
-// 1700 (six divisions, each with its own branch), and two calls of
-// timing_value 3500.
+// A cell arc's table at a load that is known before the slew: while the
+// slew's pin is waited for, the load's segment is found and how far along it
+// the load is; what is left for after the wait is the slew's segment (by
+// counting, all axis entries in flight at once), four table entries and
+// three fused multiply-adds.  In exact arithmetic the same bilinear form as
+// lut_eval's, whichever axis comes first; both lines start at the nearer end
+// of their segment.  Slew axes of up to kPrepAxis entries; others go through
+// timing_value.  After the wait an arc's two tables take about 250 cycles of
+// every gate on a path; interpolating both axes there with lut_eval took 1700
+// (six divisions, each with its own branch), and two calls of timing_value
+// 3500.  Reducing the tables to the load before the wait leaves one entry
+// pair less behind it, but costs 16 shared-memory stores a lane (240k gates
+// 1624 us against 1457) and rounds at the full value once more: slews of
+// 2k..30k gates 6.1e-8 off 64 bits, against 5.7e-8 here and 5.8e-8 with
+// lut_eval.
 constexpr int kPrepAxis = 8, kPropT = 256;
-// floats of shared memory: the values of two tables per thread, and, where
-// the library is not staged, their slew axes
-constexpr int kPrepFloats = 2 * kPrepAxis * kPropT;
 struct Prep {
-  int n;           // entries of the slew axis; 0: not prepared
-  int ax, stride;  // the axis in shared memory: ax, ax + stride, ...
-  int at;          // the values: at, at + kPropT, ...
+  int n;       // entries of the slew axis; 0: not prepared
+  int ax;      // the axis
+  int at;      // the entry of the load segment's start, first slew
+  int ds, dl;  // steps along slew and load (0: one load entry)
+  float f;     // how far along its segment the load is
+  bool end;    // measured from the segment's end
 };
 
-// which: 0, 1 of the thread's tables; prep0: where the prepared values start.
-__device__ __forceinline__ Prep prep_lut(const LutSrc& src, const Lut& m, float load, int which,
-                                         int prep0) {
+// Entry i of the library: staged in shared memory, or in global memory.
+template <bool kStaged>
+__device__ __forceinline__ float lut_at(const LutSrc& src, int i) {
   extern __shared__ float s_lut[];
-  Prep p{0, 0, 1, prep0 + which * kPrepAxis * kPropT + (int)threadIdx.x};
+  if constexpr (kStaged) return s_lut[i];
+  else return __ldg(src.gmem + i);
+}
+
+template <bool kStaged>
+__device__ __forceinline__ Prep prep_lut(const LutSrc& src, const Lut& m, float load) {
+  Prep p{0, 0, 0, 0, 0, 0.0f, false};
   const int ns = m.var == 0 ? m.n1 : m.n2, nl = m.var == 0 ? m.n2 : m.n1;
   if (m.n1 < 1 || m.n2 < 1 || m.var < 0 || ns > kPrepAxis || !(fabsf(load) < 3.402823466e+38f))
     return p;
-  const bool staged = m.off >= 0 && m.off + m.n1 + m.n2 + m.n1 * m.n2 <= src.n;
-  if (!staged && src.n > 0) return p;  // no room was left for its axis
-  const float* i1 = (staged ? src.smem : src.gmem) + m.off;
-  const float* i2 = i1 + m.n1;
-  const float* e = i2 + m.n2;  // entry of the load segment's start, first slew
-  const float* lax = m.var == 0 ? i2 : i1;
-  const int ds = m.var == 0 ? m.n2 : 1, dl = m.var == 0 ? 1 : m.n2;  // steps along slew, load
-  float f = 0.0f;
-  if (nl > 1) {
-    const int a = max(1, min(lower_bound(lax, nl, load), nl - 1));
-    f = __fdiv_rn(__fsub_rn(load, lax[a - 1]), __fsub_rn(lax[a], lax[a - 1]));
-    e += (a - 1) * dl;
-  }
-  const int next = nl > 1 ? dl : 0;
-#pragma unroll
-  for (int i = 0; i < kPrepAxis; ++i)
-    if (i < ns) {
-      const float x = e[i * ds];
-      s_lut[p.at + i * kPropT] = __fmaf_rn(f, __fsub_rn(e[i * ds + next], x), x);
-    }
-  if (staged) {
-    p.ax = m.off + (m.var == 0 ? 0 : m.n1);
-  } else {
-    const float* sax = m.var == 0 ? i1 : i2;
-    p.ax = p.at + kPrepFloats;
-    p.stride = kPropT;
-#pragma unroll
-    for (int i = 0; i < kPrepAxis; ++i)
-      if (i < ns) s_lut[p.ax + i * kPropT] = sax[i];
-  }
+  if (kStaged && (m.off < 0 || m.off + m.n1 + m.n2 + m.n1 * m.n2 > src.n)) return p;
+  const int lax = m.off + (m.var == 0 ? m.n1 : 0);
+  p.ax = m.off + (m.var == 0 ? 0 : m.n1);
+  p.at = m.off + m.n1 + m.n2;
+  p.ds = m.var == 0 ? m.n2 : 1;
   p.n = ns;
+  if (nl > 1) {
+    const int below = lower_bound((kStaged ? src.smem : src.gmem) + lax, nl, load);
+    const int a = max(1, min(below, nl - 1));
+    const float x1 = lut_at<kStaged>(src, lax + a - 1), x2 = lut_at<kStaged>(src, lax + a);
+    const float up = __fsub_rn(load, x1), down = __fsub_rn(load, x2);
+    p.dl = m.var == 0 ? 1 : m.n2;
+    p.at += (a - 1) * p.dl;
+    p.end = up > -down;
+    p.f = __fdiv_rn(p.end ? down : up, __fsub_rn(x2, x1));
+  }
   return p;
 }
 
 // Whether two prepared tables have the same slew axis.
-__device__ __forceinline__ bool same_axis(const Prep& a, const Prep& b) {
-  extern __shared__ float s_lut[];
+template <bool kStaged>
+__device__ __forceinline__ bool same_axis(const LutSrc& src, const Prep& a, const Prep& b) {
   bool same = a.n == b.n;
 #pragma unroll
   for (int i = 0; i < kPrepAxis; ++i) {
     const int k = min(i, max(min(a.n, b.n) - 1, 0));
-    same = same & (s_lut[a.ax + k * a.stride] == s_lut[b.ax + k * b.stride]);
+    same = same & (lut_at<kStaged>(src, a.ax + k) == lut_at<kStaged>(src, b.ax + k));
   }
   return same;
 }
 
 // The slew's segment on p's axis (its start, 0-based) and how far along it
-// the slew is.  No branch depends on p: half of a gate's lanes have no
-// table (the other split's, or the transitions the arc does not make), and
-// branching around them cost 1000 cycles per gate.
-__device__ __forceinline__ void prep_segment(const Prep& p, float slew, int& seg, float& t) {
-  extern __shared__ float s_lut[];
+// the slew is, from the segment's end or start.  No branch depends on p: half
+// of a gate's lanes have no table (the other split's, or the transitions the
+// arc does not make), and branching around them cost 1000 cycles per gate.
+struct Along {
+  int seg;
+  float t;
+  bool end;
+};
+template <bool kStaged>
+__device__ __forceinline__ Along prep_segment(const LutSrc& src, const Prep& p, float slew) {
+  if constexpr (!kStaged)
+    if (p.n == 0) return Along{0, 0.0f, false};  // there may be no library to read
   const int last = max(p.n - 1, 0);
   int below = 0;
 #pragma unroll
   for (int i = 0; i < kPrepAxis; ++i)
-    below += (int)(i < p.n) & (int)(s_lut[p.ax + min(i, last) * p.stride] < slew);
-  seg = max(0, min(below, last) - 1);
-  const float x1 = s_lut[p.ax + seg * p.stride];
-  const float x2 = s_lut[p.ax + min(seg + 1, last) * p.stride];
-  t = __fdiv_rn(p.n > 1 ? __fsub_rn(slew, x1) : 0.0f, p.n > 1 ? __fsub_rn(x2, x1) : 1.0f);
+    below += (int)(i < p.n) & (int)(lut_at<kStaged>(src, p.ax + min(i, last)) < slew);
+  Along s;
+  s.seg = max(0, min(below, last) - 1);
+  const float x1 = lut_at<kStaged>(src, p.ax + s.seg);
+  const float x2 = lut_at<kStaged>(src, p.ax + min(s.seg + 1, last));
+  const float up = __fsub_rn(slew, x1), down = __fsub_rn(slew, x2);
+  s.end = up > -down;
+  s.t = __fdiv_rn(p.n > 1 ? (s.end ? down : up) : 0.0f, p.n > 1 ? __fsub_rn(x2, x1) : 1.0f);
+  return s;
 }
 
-__device__ __forceinline__ float prep_value(const Prep& p, int seg, float t) {
-  extern __shared__ float s_lut[];
-  const float lo = s_lut[p.at + seg * kPropT];
-  const float hi = s_lut[p.at + (p.n > 1 ? seg + 1 : 0) * kPropT];
-  const float y = __fmaf_rn(t, __fsub_rn(hi, lo), lo);
-  return p.n > 0 ? y : nanf("");
+template <bool kStaged>
+__device__ __forceinline__ float prep_value(const LutSrc& src, const Prep& p, const Along& s) {
+  if constexpr (!kStaged)
+    if (p.n == 0) return nanf("");
+  const int i0 = p.at + s.seg * p.ds, i1 = i0 + (p.n > 1 ? p.ds : 0);
+  const float a0 = lut_at<kStaged>(src, i0), b0 = lut_at<kStaged>(src, i0 + p.dl);
+  const float a1 = lut_at<kStaged>(src, i1), b1 = lut_at<kStaged>(src, i1 + p.dl);
+  // the table and its step along the load at either end of the slew's segment
+  const float e0 = p.end ? b0 : a0, e1 = p.end ? b1 : a1;
+  const float g0 = __fsub_rn(b0, a0), g1 = __fsub_rn(b1, a1);
+  const float e = __fmaf_rn(s.t, __fsub_rn(e1, e0), s.end ? e1 : e0);
+  const float g = __fmaf_rn(s.t, __fsub_rn(g1, g0), s.end ? g1 : g0);
+  return p.n > 0 ? __fmaf_rn(p.f, g, e) : nanf("");
 }
 
 // RC node of a net arc's sink (arc_node: its local id in the net) as a
@@ -403,11 +417,11 @@ struct Visit {
 // and _fprop_test.  Lane j of a pass takes fanin arc j/8 and the combination
 // (el, frf, trf) = bits (2, 1, 0) of j; its slew and arrival candidates go to
 // output corner (el, trf).  Returns false if a wait gave up.
-template <class AfterF>
+template <bool kStaged, class AfterF>
 __device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const LutSrc& lutd,
-                                           int prep0, const Visit& me, int lane, float* at,
-                                           float* slew, float* rat, float* arc_delay,
-                                           float* test_rat, GridCtl* ctl, AfterF after) {
+                                           const Visit& me, int lane, float* at, float* slew,
+                                           float* rat, float* arc_delay, float* test_rat,
+                                           GridCtl* ctl, AfterF after) {
   const otg_prop_graph& g = G_.g;
   const int v = me.v;
   const int el = (lane >> 2) & 1, frf = (lane >> 1) & 1, trf = lane & 1;
@@ -430,8 +444,7 @@ __device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const L
     const bool cell = R.w != kNetRec, thru = cell && R.y != kOwnRec;
     float d = nanf(""), so = nanf(""), imp = nanf("");
     Lut ls = no_lut(), ld = no_lut();
-    Prep ps, pd;
-    ps.n = pd.n = 0;
+    Prep ps{}, pd{};
     bool one_axis = true, slow = false;
     float load = 0.0f;
     // the sink whose Elmore delay and impulse the lane adds: a net arc's
@@ -447,9 +460,9 @@ __device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const L
       ls = timing_lut(G_, t, 1, frf, trf);
       ld = timing_lut(G_, t, 0, frf, trf);
       if (R.w >= 0 && t >= 0) load = __ldg(G_.rc.load + 4 * (size_t)R.w + c_out);
-      ps = prep_lut(lutd, ls, load, 0, prep0);
-      pd = prep_lut(lutd, ld, load, 1, prep0);
-      one_axis = ps.n == 0 || pd.n == 0 || same_axis(ps, pd);
+      ps = prep_lut<kStaged>(lutd, ls, load);
+      pd = prep_lut<kStaged>(lutd, ld, load);
+      one_axis = ps.n == 0 || pd.n == 0 || same_axis<kStaged>(lutd, ps, pd);
       slow = (ls.n1 >= 0 && ps.n == 0) || (ld.n1 >= 0 && pd.n == 0);
     }
     // what the code after the wait reads is loaded here (the compiler may
@@ -477,12 +490,10 @@ __device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const L
       so = none(si) ? nanf("") : timing_value(lutd, ls, si, load);
       d = none(si) ? nanf("") : timing_value(lutd, ld, si, load);
     } else {
-      int seg;
-      float t;
-      prep_segment(ps, si, seg, t);
-      so = prep_value(ps, seg, t);
-      if (!one_axis) prep_segment(pd, si, seg, t);
-      d = prep_value(pd, seg, t);
+      Along x = prep_segment<kStaged>(lutd, ps, si);
+      so = prep_value<kStaged>(lutd, ps, x);
+      if (!one_axis) x = prep_segment<kStaged>(lutd, pd, si);
+      d = prep_value<kStaged>(lutd, pd, x);
     }
     if (cell) arr = none(fa) || none(d) ? nanf("") : __fadd_rn(d, fa);
     if (on) {
@@ -772,7 +783,7 @@ __global__ void prop_init_kernel(float4* at, float4* slew, int num_pins, GridCtl
 // pins, more warps count (four CTAs, 64 registers: 240k gates 1.34 ms
 // against 1.86 with two), where it has few, the chain of waits does (two,
 // 103 registers, no spills on it: 2k gates 194 us against 216).
-template <int kCtas>
+template <int kCtas, bool kStaged>
 __global__ void __launch_bounds__(kPropT, kCtas)
     prop_kernel(G G_, const int* order, const int* fwd_order, int num_pins, float* at, float* slew,
                 float* rat, float* slack, float* arc_delay, float* test_rat, GridCtl* ctl,
@@ -784,7 +795,6 @@ __global__ void __launch_bounds__(kPropT, kCtas)
   for (int i = threadIdx.x; i < lut_smem; i += blockDim.x) s_lut[i] = __ldg(G_.g.lut_data + i);
   __syncthreads();
   const LutSrc lutd{s_lut, lut_smem, G_.g.lut_data};
-  const int prep0 = lut_smem;  // the prepared tables follow
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int W = (gridDim.x * blockDim.x) >> 5;
@@ -816,8 +826,8 @@ __global__ void __launch_bounds__(kPropT, kCtas)
       const int v2 = pin(list, down, j + 2 * W);
       range(G_.g.fanin_start, next);
       if (me.v >= 0)
-        ok = fprop_warp(G_, rec, lutd, prep0, me, lane, at, slew, rat, arc_delay, test_rat, ctl,
-                        [&] { first(next); });
+        ok = fprop_warp<kStaged>(G_, rec, lutd, me, lane, at, slew, rat, arc_delay, test_rat, ctl,
+                                 [&] { first(next); });
       else
         first(next);
       me = next;
@@ -841,11 +851,6 @@ size_t align256p(size_t x) { return (x + 255) & ~(size_t)255; }
 // allow; a library with three drive strengths of its combinational cells
 // takes about 33 KB).
 constexpr int kLutSmemFloats = 10240;
-
-// Dynamic shared memory of the kernel with lut_smem floats of staged tables.
-size_t prop_smem(int lut_smem) {
-  return 4 * ((size_t)lut_smem + kPrepFloats * (lut_smem ? 1 : 2));
-}
 
 // Up to this many pins per warp at two CTAs per SM, those are launched
 // (2k gates have 2, a 6k-gate block 8: 666 us against 718; 60k gates 69:
@@ -916,15 +921,16 @@ static otg_status propagate_impl(const otg_prop_graph* g, const otg_prop_rc* rc,
   otg::PropDev& d = otg::g_pdev[dev & 63];
   if (!d.init) {
     cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
-    for (auto k : {otg::prop_kernel<2>, otg::prop_kernel<4>})
+    for (auto k : {otg::prop_kernel<2, true>, otg::prop_kernel<4, true>})
       cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)otg::prop_smem(otg::kLutSmemFloats));
+                           4 * otg::kLutSmemFloats);
     d.init = true;
   }
   int lut_smem = g->num_lut_data > 0 && g->num_lut_data <= otg::kLutSmemFloats ? g->num_lut_data : 0;
-  const size_t smem = otg::prop_smem(lut_smem);
+  const size_t smem = 4 * (size_t)lut_smem;
   const bool few = P <= otg::kFewPins * 2 * d.sms * (otg::kPropT / 32);
-  auto kern = few ? otg::prop_kernel<2> : otg::prop_kernel<4>;
+  auto kern = lut_smem ? (few ? otg::prop_kernel<2, true> : otg::prop_kernel<4, true>)
+                       : (few ? otg::prop_kernel<2, false> : otg::prop_kernel<4, false>);
   long long known = d.occ[few].load(std::memory_order_relaxed);
   if ((known >> 32) != lut_smem + 1) {
     int o = 0;
