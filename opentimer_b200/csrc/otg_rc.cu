@@ -1027,8 +1027,9 @@ __global__ void __launch_bounds__(T, TILE ? 1024 / T : 1) rc_block_kernel(RcJob 
 // walks the same items without a shared fetch.  A class of more than
 // `few` items is left to the one-CTA-per-net kernel (many huge nets keep
 // every SM busy on their own; a few finish sooner on clusters).
-template <int T, int K>
-__global__ void __launch_bounds__(T) rc_cluster_kernel(RcJob job, const int* list,
+// kCtas: CTAs per SM its registers allow.
+template <int T, int K, int kCtas>
+__global__ void __launch_bounds__(T, kCtas) rc_cluster_kernel(RcJob job, const int* list,
                                                        const int* count, char* gws,
                                                        size_t ws_stride, int few) {
   __shared__ int sh[96];
@@ -1283,32 +1284,44 @@ int huge_ctas(int sms, size_t stride) {
 
 // The huge-net path: one CTA per net, and clusters of S CTAs of 512
 // threads per net.  Both are launched; the device-side count of huge nets
-// picks one: clusters for at most kClusterNetsPerCluster nets per cluster,
-// one CTA per net for more.  S defaults to 8 (the portable cluster size),
-// capped by what the device places; OTG_RC_HUGE_CLUSTER=2|4|8|16 asks for
-// another size, =1 turns the clusters off.
-constexpr int kHugeT = 512, kHugeK = 8;
-constexpr int kClusterNetsPerCluster = 2;
+// picks one: clusters for at most `few` of them, one CTA per net for more.
+// S defaults to 8 (the portable cluster size), 16 for a pass of at most
+// kLoneNets nets (one net of 20,000 nodes: 245 us against 333; eight of
+// 5k..20k: 410 against 374), capped by what the device places;
+// OTG_RC_HUGE_CLUSTER=2|4|8|16 asks for another size, =1 turns the clusters
+// off.  Where a pass may have more nets than clusters of one CTA per SM
+// find room for, two CTAs share an SM, on half the registers: one net takes
+// 6% longer and 24 of 5k..20k nodes 423 us instead of 528, 40 of them 566
+// instead of 1290.
+constexpr int kHugeT = 512, kHugeK = 8, kPairK = 4;
+constexpr int kLoneNets = 4, kTwoRounds = 8000;
 struct HugePlan {
   int S = 1;            // CTAs per cluster (1: no cluster launch)
+  bool pair = false;    // two CTAs per SM
   int clusters = 0;     // clusters launched, one workspace slice each
   size_t stride_c = 0;  // bytes per cluster slice
+  int few = 0;          // nets that the clusters take
   int ctas = 0;         // CTAs of the one-CTA-per-net launch, one slice each
   size_t stride = 0;    // bytes per slice of that launch
-  size_t bytes() const { return stride * (size_t)ctas + stride_c * (size_t)clusters; }
+  size_t bytes = 0;     // of the slices, the two launches' in the same place
 };
 
-int max_clusters(int S) {  // clusters of S CTAs the device holds at once (0: none)
+using ClusterKernel = decltype(&rc_cluster_kernel<kHugeT, kHugeK, 1>);
+ClusterKernel cluster_kernel(bool pair) {
+  return pair ? rc_cluster_kernel<kHugeT, kPairK, 2> : rc_cluster_kernel<kHugeT, kHugeK, 1>;
+}
+
+int max_clusters(int S, bool pair) {  // clusters of S CTAs the device holds at once (0: none)
   static std::mutex mu;
-  static int cache[64][5];
-  static bool done[64][5];
+  static int cache[64][5][2];
+  static bool done[64][5][2];
   int d = 0;
   cudaGetDevice(&d);
   int si = 0;
   while ((1 << si) < S && si < 4) ++si;
   std::lock_guard<std::mutex> lk(mu);
-  if (!done[d & 63][si]) {
-    auto kern = rc_cluster_kernel<kHugeT, kHugeK>;
+  if (!done[d & 63][si][pair]) {
+    auto kern = cluster_kernel(pair);
     int nc = 0;
     if (S > 8) cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg = {};
@@ -1323,29 +1336,45 @@ int max_clusters(int S) {  // clusters of S CTAs the device holds at once (0: no
     cfg.numAttrs = 1;
     if (cudaOccupancyMaxActiveClusters(&nc, (const void*)kern, &cfg) != cudaSuccess) nc = 0;
     cudaGetLastError();
-    cache[d & 63][si] = nc;
-    done[d & 63][si] = true;
+    cache[d & 63][si][pair] = nc;
+    done[d & 63][si][pair] = true;
   }
-  return cache[d & 63][si];
+  return cache[d & 63][si][pair];
 }
 
-HugePlan huge_plan(int max_net_nodes, int sms) {
+// For a pass of at most `nets` nets.
+HugePlan huge_plan(int max_net_nodes, int sms, int nets) {
   HugePlan h;
   h.stride = align256(rc_layout(max_net_nodes, kHugeT, kHugeK, 4).total);
   h.ctas = huge_ctas(sms, h.stride);
-  int S = 8;
-  if (const char* e = std::getenv("OTG_RC_HUGE_CLUSTER")) S = std::atoi(e);
-  int s2 = 1;
-  while (s2 * 2 <= std::min(std::max(S, 1), 16)) s2 *= 2;
-  S = s2;
+  h.bytes = h.stride * (size_t)h.ctas;
+  int asked = 8;
+  const char* env = std::getenv("OTG_RC_HUGE_CLUSTER");
+  if (env) asked = std::min(std::max(std::atoi(env), 1), 16);
+  int S = 1;
+  while (S * 2 <= asked) S *= 2;
   int ncl = 0;
-  while (S > 1 && (ncl = max_clusters(S)) < 1) S /= 2;
-  if (S > 1) {
-    h.S = S;
-    h.stride_c = align256(rc_layout(max_net_nodes, kHugeT, kHugeK, 4, S).total);
-    const size_t cap = ((size_t)4 << 30) / std::max<size_t>(h.stride_c, 1);
-    h.clusters = (int)std::max<size_t>(1, std::min<size_t>((size_t)ncl, cap));
+  while (S > 1 && (ncl = max_clusters(S, false)) < 1) S /= 2;
+  if (S == 1) return h;
+  auto slice = [&](int s) { return align256(rc_layout(max_net_nodes, kHugeT, kHugeK, 4, s).total); };
+  auto fit = [](size_t bytes, size_t room) { return (int)std::max<size_t>(1, room / bytes); };
+  h.stride_c = slice(S);
+  // the size does not depend on `nets`: a workspace serves any smaller pass
+  h.bytes += h.stride_c * (size_t)std::min(ncl, fit(h.stride_c, (size_t)4 << 30));
+  if (!env && S == 8 && nets <= kLoneNets && slice(16) <= h.bytes && max_clusters(16, false) >= 1) {
+    S = 16;
+    ncl = max_clusters(16, false);
+    h.stride_c = slice(16);
+  } else if (nets > ncl && max_clusters(S, true) > ncl) {
+    h.pair = true;
+    ncl = max_clusters(S, true);
   }
+  h.S = S;
+  h.clusters = std::min(ncl, fit(h.stride_c, h.bytes));
+  // two rounds of clusters still beat one CTA per net (36 nets of 12,000
+  // nodes: 602 us against 939), not for the smallest of them (40 of
+  // 5,000..6,000: 430 against 394)
+  h.few = h.clusters * (max_net_nodes > kTwoRounds ? 2 : 1);
   return h;
 }
 
@@ -1362,9 +1391,9 @@ size_t rc_workspace_bytes_for(const RcTune& t, int num_nets, int max_net_nodes, 
   *off_huge = o;
   *huge_stride = 0;
   if (max_net_nodes > c.nmax[6]) {
-    const HugePlan h = huge_plan(max_net_nodes, sms);
+    const HugePlan h = huge_plan(max_net_nodes, sms, std::max(num_nets, 1));
     *huge_stride = h.stride;
-    o += h.bytes();
+    o += h.bytes;
   }
   return o;
 }
@@ -1545,15 +1574,13 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
   }
   // Largest nets first so the long tail overlaps the small ones.
   if (err == cudaSuccess && max_net_nodes > cls.nmax[6]) {
-    const HugePlan h = huge_plan(max_net_nodes, di.sms);
-    const int few = h.S > 1 ? kClusterNetsPerCluster * h.clusters : 0;
+    const HugePlan h = huge_plan(max_net_nodes, di.sms, cap);
     cudaStream_t hs = next_stream();
     err = chain_launch(rc_block_kernel<kHugeT, kHugeK, int, false>, h.ctas, kHugeT, 0, 1, chained,
-                       hs, job, L(7), counters + 7, work + 7, ws + off_huge, stride, few);
+                       hs, job, L(7), counters + 7, work + 7, ws + off_huge, stride, h.few);
     if (err == cudaSuccess && h.S > 1)
-      err = chain_launch(rc_cluster_kernel<kHugeT, kHugeK>, h.clusters * h.S, kHugeT, 0, h.S,
-                         nside == 0, hs, job, L(7), counters + 7,
-                         ws + off_huge + stride * (size_t)h.ctas, h.stride_c, few);
+      err = chain_launch(cluster_kernel(h.pair), h.clusters * h.S, kHugeT, 0, h.S, nside == 0, hs,
+                         job, L(7), counters + 7, ws + off_huge, h.stride_c, h.few);
   }
   for (int c = tn.num; c >= 1 && err == cudaSuccess; --c) {
     if (max_net_nodes <= cls.nmax[c - 1]) continue;
