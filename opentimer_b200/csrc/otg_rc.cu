@@ -1510,9 +1510,13 @@ bool forest_ok(const otg_rc_forest* f) {
 
 }  // namespace
 
-// CTAs of the small-net kernel: one warp and eight nets each at a time.
-int small_ctas(int nets, int sms) {
-  return std::max(1, std::min((nets + 7) / 8, kSmallCtas * sms));
+// CTAs of the small-net kernel, one warp each: as many as its nets take in
+// one go, eight of up to 16 nodes, four of larger ones (with eight, 2,243 nets
+// of 2..24 nodes took two: 30.5 us against 18.5), and one net each where there
+// are few (300 nets of 2..24 nodes 16.8 us, of 2..32 20.6 against 22.6).
+int small_ctas(int nets, int max_net_nodes, int sms) {
+  const int k = max_net_nodes <= kSmallCells / 8 ? 8 : (nets > 4 * sms ? 4 : 1);
+  return std::max(1, std::min((nets + k - 1) / k, kSmallCtas * sms));
 }
 
 // Launches the fused pass over the items of `job` (at most `cap` of them).
@@ -1543,7 +1547,7 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
   // every net is small: no classes to sort into (sorting 250,000 nets takes
   // 9 us, and a call of 64 nets a third of its launches)
   if (max_net_nodes <= kSmallMax) {
-    rc_small_kernel<<<small_ctas(cap, di.sms), 32, 0, stream>>>(
+    rc_small_kernel<<<small_ctas(cap, max_net_nodes, di.sms), 32, 0, stream>>>(
         job, nullptr, nullptr, cap, max_net_nodes, status);
     count_launch();
     if (cudaGetLastError() != cudaSuccess) return OTG_ERR_CUDA;
@@ -1591,7 +1595,7 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
   }
   if (err == cudaSuccess) {
     cudaStream_t st = next_stream();
-    err = chain_launch(rc_small_kernel, small_ctas(cap, di.sms), 32, 0, 1, chained, st, job, L(0),
+    err = chain_launch(rc_small_kernel, small_ctas(cap, max_net_nodes, di.sms), 32, 0, 1, chained, st, job, L(0),
                        counters + 0, cap, max_net_nodes, status);
   }
   // join (also after a failed launch, so a capture is never left unjoined)
