@@ -1198,9 +1198,12 @@ RcTune default_tune(int smem_budget, long long nets, int max_net_nodes, int sms)
     int nmax;
     Shape s;
   };
-  // 2496: the most that leave room for two CTAs of 512 threads on an SM
+  // 1232 and 2496: the most that leave room for four CTAs of 256 threads and
+  // two of 512 on an SM (164,380 nets of 2..1500 nodes: 4.87 ms, 5.06 with
+  // 1024 for 1232; 100,000 of 2..4096: 7.01 and 7.13, 7.38 with 256 threads
+  // up to 2496)
   constexpr Row many[] = {{128, {64, 4}},  {256, {64, 8}},   {512, {128, 8}},
-                          {1024, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
+                          {1232, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
   constexpr Row some[] = {{512, {128, 8}}, {1024, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
   const Row few[] = {{512, {max_net_nodes <= 128 ? 128 : 256, 4}}, {1024, {512, 4}}, {0, {1024, 4}}};
   RcTune t;

@@ -42,3 +42,21 @@ def test_warp_per_net_same_bits(cuda):
         otg.set_tuning(None)
     for k in OUT:
         assert np.array_equal(one[k], two[k]), k
+
+
+# the class table depends on the number of nets: one for up to 8 an SM, one
+# for up to 20, one for more (1,184 and 2,960 nets on 148 SMs)
+@pytest.mark.parametrize("nets", [40, 1500, 3100])
+def test_class_tables(cuda, nets):
+    edges = [33, 64, 128, 129, 256, 257, 512, 513, 1024, 1025, 1232, 1233, 2496, 2497, 4888, 4889]
+    sizes = edges + [2 + i % 60 for i in range(nets - len(edges))]
+    f = rcgen.forest(nets, sizes)
+    got = run(cuda, f)
+    st, e, n2b, pid, _ = O.bfs(f)
+    assert st == 0
+    assert np.array_equal(got["node2bfs"], n2b) and np.array_equal(got["pid"], pid)
+    assert np.array_equal(got["edges"], e)
+    st, ref = O.elmore_f64(f)
+    assert st == 0
+    for q, r in zip(["load", "delay", "ldelay", "impulse"], ref):
+        assert elmore_err(f.nodes_start, bfs_local(f.nodes_start, n2b, got[q]), r) <= 1.0, q
