@@ -22,7 +22,8 @@
 //     depth, DFS preorder and subtree sizes, a stable radix sort by depth
 //     yields the reference's BFS slots, and Elmore runs as two exact int64
 //     fixed-point scans up the preorder (subtree sums: load, ldelay) and two
-//     down the Euler tour (path sums: delay, beta).
+//     path sums (delay, beta): down the Euler tour, or in the tile kernel as
+//     the prefix over the preorder less the one over the postorder.
 //
 // BFS order is bit-exact with the reference: (distance asc, local id desc).
 #include <cooperative_groups.h>
