@@ -782,7 +782,7 @@ __global__ void prop_init_kernel(float4* at, float4* slew, int num_pins, GridCtl
 // w, w + W, ... of each pass.  kCtas CTAs per SM: where a warp has many
 // pins, more warps count (four CTAs, 64 registers: 240k gates 1.34 ms
 // against 1.86 with two), where it has few, the chain of waits does (two,
-// 103 registers, no spills on it: 2k gates 194 us against 216).
+// 90 registers, no spills on it: 2k gates 194 us against 216).
 template <int kCtas, bool kStaged>
 __global__ void __launch_bounds__(kPropT, kCtas)
     prop_kernel(G G_, const int* order, const int* fwd_order, int num_pins, float* at, float* slew,
