@@ -226,31 +226,32 @@ __device__ __forceinline__ bool same_axis(const LutSrc& src, const Prep& a, cons
   return same;
 }
 
-// The slew's segment on p's axis (its start, 0-based) and how far along it
-// the slew is, from the segment's end or start.  No branch depends on p: half
-// of a gate's lanes have no table (the other split's, or the transitions the
-// arc does not make), and branching around them cost 1000 cycles per gate.
+// The slew's segment on an axis of n entries from ax (its start, 0-based) and
+// how far along it the slew is, from the segment's end or start.  No branch
+// depends on n, which is 0 without a table: half of a gate's lanes have none
+// (the other split's, or the transitions the arc does not make), and branching
+// around them cost 1000 cycles per gate.
 struct Along {
   int seg;
   float t;
   bool end;
 };
 template <bool kStaged>
-__device__ __forceinline__ Along prep_segment(const LutSrc& src, const Prep& p, float slew) {
+__device__ __forceinline__ Along prep_segment(const LutSrc& src, int n, int ax, float slew) {
   if constexpr (!kStaged)
-    if (p.n == 0) return Along{0, 0.0f, false};  // there may be no library to read
-  const int last = max(p.n - 1, 0);
+    if (n == 0) return Along{0, 0.0f, false};  // there may be no library to read
+  const int last = max(n - 1, 0);
   int below = 0;
 #pragma unroll
   for (int i = 0; i < kPrepAxis; ++i)
-    below += (int)(i < p.n) & (int)(lut_at<kStaged>(src, p.ax + min(i, last)) < slew);
+    below += (int)(i < n) & (int)(lut_at<kStaged>(src, ax + min(i, last)) < slew);
   Along s;
   s.seg = max(0, min(below, last) - 1);
-  const float x1 = lut_at<kStaged>(src, p.ax + s.seg);
-  const float x2 = lut_at<kStaged>(src, p.ax + min(s.seg + 1, last));
+  const float x1 = lut_at<kStaged>(src, ax + s.seg);
+  const float x2 = lut_at<kStaged>(src, ax + min(s.seg + 1, last));
   const float up = __fsub_rn(slew, x1), down = __fsub_rn(slew, x2);
   s.end = up > -down;
-  s.t = __fdiv_rn(p.n > 1 ? (s.end ? down : up) : 0.0f, p.n > 1 ? __fsub_rn(x2, x1) : 1.0f);
+  s.t = __fdiv_rn(n > 1 ? (s.end ? down : up) : 0.0f, n > 1 ? __fsub_rn(x2, x1) : 1.0f);
   return s;
 }
 
@@ -490,9 +491,10 @@ __device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const L
       so = none(si) ? nanf("") : timing_value(lutd, ls, si, load);
       d = none(si) ? nanf("") : timing_value(lutd, ld, si, load);
     } else {
-      Along x = prep_segment<kStaged>(lutd, ps, si);
+      // on the slew table's axis, or the delay table's where there is no other
+      Along x = prep_segment<kStaged>(lutd, ps.n ? ps.n : pd.n, ps.n ? ps.ax : pd.ax, si);
       so = prep_value<kStaged>(lutd, ps, x);
-      if (!one_axis) x = prep_segment<kStaged>(lutd, pd, si);
+      if (!one_axis) x = prep_segment<kStaged>(lutd, pd.n, pd.ax, si);
       d = prep_value<kStaged>(lutd, pd, x);
     }
     if (cell) arr = none(fa) || none(d) ? nanf("") : __fadd_rn(d, fa);
