@@ -235,17 +235,24 @@ struct Along {
   int seg;
   float t;
   bool end;
+  bool line;  // the entries below the slew are the axis' first ones
 };
 template <bool kStaged>
 __device__ __forceinline__ Along prep_segment(const LutSrc& src, int n, int ax, float slew) {
   if constexpr (!kStaged)
-    if (n == 0) return Along{0, 0.0f, false};  // there may be no library to read
+    if (n == 0) return Along{0, 0.0f, false, true};  // there may be no library to read
   const int last = max(n - 1, 0);
   int below = 0;
+  bool all = true, gap = false;
 #pragma unroll
-  for (int i = 0; i < kPrepAxis; ++i)
-    below += (int)(i < n) & (int)(lut_at<kStaged>(src, ax + min(i, last)) < slew);
+  for (int i = 0; i < kPrepAxis; ++i) {
+    const bool is = (i < n) & (lut_at<kStaged>(src, ax + min(i, last)) < slew);
+    below += (int)is;
+    gap = gap | (is & !all);
+    all = is;
+  }
   Along s;
+  s.line = !gap;
   s.seg = max(0, min(below, last) - 1);
   const float x1 = lut_at<kStaged>(src, ax + s.seg);
   const float x2 = lut_at<kStaged>(src, ax + min(s.seg + 1, last));
@@ -486,16 +493,27 @@ __device__ __forceinline__ bool fprop_warp(const G& G_, const int4* rec, const L
     }
     if (!cell) {
       so = sink;
-    } else if (slow || !(fabsf(si) < 3.402823466e+38f)) {
-      // rare: not one straight line for all of the warp's arcs
-      so = none(si) ? nanf("") : timing_value(lutd, ls, si, load);
-      d = none(si) ? nanf("") : timing_value(lutd, ld, si, load);
     } else {
-      // on the slew table's axis, or the delay table's where there is no other
-      Along x = prep_segment<kStaged>(lutd, ps.n ? ps.n : pd.n, ps.n ? ps.ax : pd.ax, si);
-      so = prep_value<kStaged>(lutd, ps, x);
-      if (!one_axis) x = prep_segment<kStaged>(lutd, pd.n, pd.ax, si);
-      d = prep_value<kStaged>(lutd, pd, x);
+      bool line = !slow && fabsf(si) < 3.402823466e+38f;
+      if (line) {
+        // on the slew table's axis, or the delay table's where there is no other
+        Along x = prep_segment<kStaged>(lutd, ps.n ? ps.n : pd.n, ps.n ? ps.ax : pd.ax, si);
+        line = x.line;
+        so = prep_value<kStaged>(lutd, ps, x);
+        if (!one_axis) {
+          x = prep_segment<kStaged>(lutd, pd.n, pd.ax, si);
+          line = line && x.line;
+        }
+        d = prep_value<kStaged>(lutd, pd, x);
+        line = line && (ps.n == 0 || isfinite(so)) && (pd.n == 0 || isfinite(d));
+      }
+      // rare: not one straight line for all of the warp's arcs, an axis out of
+      // order, or a look-up that met a segment of no length or an entry that is
+      // not finite, where the rule's own cases count (a query on an entry)
+      if (!line) {
+        so = none(si) ? nanf("") : timing_value(lutd, ls, si, load);
+        d = none(si) ? nanf("") : timing_value(lutd, ld, si, load);
+      }
     }
     if (cell) arr = none(fa) || none(d) ? nanf("") : __fadd_rn(d, fa);
     if (on) {

@@ -1,5 +1,6 @@
-"""Propagation through timing records that lack a table, against the look-up
-rule in 64 bits.
+"""Propagation through timing records that lack a table, and through tables
+at the edges of the look-up rule (repeated axis entries, entries that are not
+finite, axes out of order), against the rule itself in 64 bits.
 
 The design is that of test_prop_paths_gpu.py: one driver whose net has F
 sinks, each the input of a cell with one output, a primary output."""
@@ -129,4 +130,34 @@ def test_missing_tables(cuda, luts, var, pad):
     tables = [table(rng, 0.02 + 0.03 * np.arange(7), lo * (0.5 + 0.4 * np.arange(7)), var)
               for _ in range(4)]
     record = [0, 0, 0, *luts, -1, -1]
+    expect_and_check(graph(cuda, record, tables, pad), b, record, tables)
+
+
+@pytest.mark.parametrize("axis", ["slew", "load"])
+@pytest.mark.parametrize("form", ["repeated first", "all repeated", "repeated, query above",
+                                  "repeated, query below", "descending", "nan inside",
+                                  "infinite beside", "infinite around"])
+@pytest.mark.parametrize("pad", [0, 12000], ids=["staged", "global"])
+def test_lookup_edges(cuda, axis, form, pad):
+    rng = np.random.default_rng(3)
+    b = net(cuda)
+    load = b.load.cpu().numpy()[0]
+    plain = [table(rng, 0.02 + 0.03 * np.arange(4), load[0] * (0.5 + 0.4 * np.arange(5)), 0)] * 4
+    record = [0, 0, 0, 0, 1, 2, 3, -1, -1]
+    # the first sink's own slew (as the device rounds it) and the net's load
+    q = graph(cuda, record, plain, pad).propagate(b).result()["slew"][1, 2] \
+        if axis == "slew" else load[2]
+    ax = {"repeated first": [q, q, 2 * q, 3 * q], "all repeated": [q, q],
+          "repeated, query above": [0.5 * q, 0.5 * q], "repeated, query below": [2 * q, 2 * q, 3 * q],
+          "descending": [3 * q, 2 * q, 1.5 * q, 0.7 * q, 0.5 * q],
+          "nan inside": [0.1 * q, 0.2 * q, np.nan, 0.4 * q, 0.5 * q, 0.9 * q, 2 * q],
+          "infinite beside": [q, 2 * q, 4 * q],
+          "infinite around": [0.2 * q, 1.1 * q, 2 * q]}[form]
+    other = load[0] * (0.5 + 0.4 * np.arange(5)) if axis == "slew" else 0.02 + 0.03 * np.arange(5)
+    sax, lax = (ax, other) if axis == "slew" else (other, ax)
+    tables = [table(rng, sax, lax, k & 1) for k in range(4)]
+    if form.startswith("infinite"):
+        for t in tables:  # at entry 1 of the axis in question
+            along = t[2] if (axis == "slew") == (t[3] == 0) else t[2].T
+            along[1] = np.inf
     expect_and_check(graph(cuda, record, tables, pad), b, record, tables)
