@@ -446,20 +446,27 @@ __global__ void __launch_bounds__(LT, 1) levelize_grid_kernel(LvArgs a) {
 //
 // Pins by level - 1 (level 0 is the seed, in the caller's order), stable in
 // the pin index: digits of kDigitBits, each by a histogram per tile of
-// consecutive items, a scan and a scatter.  Graphs of more than kDigits + 1
-// levels take a second digit, whose kernels return at once otherwise.
+// consecutive items, a scan and a scatter.  A pass whose digit is 0 for every
+// level is left out: its kernels return at once, and where the graph has too
+// few pins for so many levels, they are not launched.
 constexpr int kDigitBits = 10, kDigits = 1 << kDigitBits, kMaxTiles = 256, ST = 1024;
 
 struct LvSort {
   int per;      // items per tile
   int tiles;
   int* hist;    // [kDigits][tiles]
-  int* first;   // the pins by the first digit, where there are two
+  int* part;    // two lists of n pins: sorted by the digits so far, by pass
   int* num;     // their number
 };
 
+// Whether a pass has nothing to sort: the digit of the highest level - 1,
+// and all above it, are 0.
+__host__ __device__ __forceinline__ bool sort_skip(int levels, int pass) {
+  return pass > 0 && ((long long)levels - 2) >> (kDigitBits * pass) <= 0;
+}
+
 // Item i of a pass and its digit (-1: not an item): the pins in index order
-// (pass 0), or the first pass's output.
+// (pass 0), or the pass before's output.
 __device__ __forceinline__ int sort_item(const LvArgs& a, const LvSort& s, int pass, int i,
                                          int& v) {
   if (pass == 0) {
@@ -468,17 +475,14 @@ __device__ __forceinline__ int sort_item(const LvArgs& a, const LvSort& s, int p
     return l > 0 ? (l - 1) & (kDigits - 1) : -1;
   }
   if (i >= *s.num) return -1;
-  v = s.first[i];
-  return ((a.level[v] - 1) >> kDigitBits) & (kDigits - 1);
-}
-__device__ __forceinline__ bool sort_skip(const LvArgs& a, int pass) {
-  return pass == 1 && a.ctl->levels <= kDigits + 1;
+  v = s.part[(size_t)((pass - 1) & 1) * a.n + i];
+  return ((a.level[v] - 1) >> (kDigitBits * pass)) & (kDigits - 1);
 }
 
 __global__ void __launch_bounds__(ST) levelize_hist(LvArgs a, LvSort s, int pass) {
   __shared__ int h[kDigits];
   asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
-  if (sort_skip(a, pass)) return;
+  if (sort_skip(a.ctl->levels, pass)) return;
   for (int d = threadIdx.x; d < kDigits; d += ST) h[d] = 0;
   __syncthreads();
   const int b = blockIdx.x * s.per;
@@ -496,7 +500,7 @@ __global__ void __launch_bounds__(ST) levelize_hist(LvArgs a, LvSort s, int pass
 __global__ void __launch_bounds__(kDigits) levelize_scan(LvArgs a, LvSort s, int pass) {
   __shared__ int wsum[kDigits / 32];
   asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
-  if (sort_skip(a, pass)) return;
+  if (sort_skip(a.ctl->levels, pass)) return;
   const int d = threadIdx.x, lane = d & 31, w = d >> 5;
   int* row = s.hist + d * s.tiles;
   int sum = 0;
@@ -549,8 +553,8 @@ __global__ void __launch_bounds__(ST) levelize_scatter(LvArgs a, LvSort s, int p
   uint16_t* cnt = (uint16_t*)lv_sm;                  // [warp][digit], then the warps' bases
   int* base = (int*)(cnt + (ST / 32) * kDigits);     // [digit] the tile's base
   asm volatile("griddepcontrol.launch_dependents;\n griddepcontrol.wait;" ::: "memory");
-  if (sort_skip(a, pass)) return;
-  const bool last = pass == 1 || a.ctl->levels <= kDigits + 1;
+  if (sort_skip(a.ctl->levels, pass)) return;
+  const bool last = sort_skip(a.ctl->levels, pass + 1);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   for (int i = threadIdx.x; i < (ST / 32) * kDigits / 2; i += ST) ((unsigned*)cnt)[i] = 0u;
   for (int d = threadIdx.x; d < kDigits; d += ST) base[d] = s.hist[d * s.tiles + blockIdx.x];
@@ -576,7 +580,7 @@ __global__ void __launch_bounds__(ST) levelize_scatter(LvArgs a, LvSort s, int p
     }
   }
   __syncthreads();
-  int* out = last ? a.order : s.first;
+  int* out = last ? a.order : s.part + (size_t)(pass & 1) * a.n;
   const int off = last ? a.first_size : 0;
   for (int i = 0; i < per; i += 32) {
     int v;
@@ -597,7 +601,7 @@ __global__ void __launch_bounds__(ST) levelize_scatter(LvArgs a, LvSort s, int p
 // them.
 __global__ void levelize_ends(LvArgs a, LvSort s) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (sort_skip(a, 1)) return;
+  if (sort_skip(a.ctl->levels, 1)) return;
   const int end = min(a.first_size + *s.num, a.n);
   for (int p = a.first_size + blockIdx.x * blockDim.x + threadIdx.x; p < end;
        p += gridDim.x * blockDim.x) {
@@ -832,20 +836,20 @@ otg_status otg_levelize(int32_t n, int32_t num_edges, const int32_t* fanin_start
   }
   otg::LvSort s = otg::lv_tiles(n);
   s.hist = (int*)(ws + l.hist);
-  s.first = (int*)(ws + l.packed);  // the records have been read
+  s.part = (int*)(ws + l.packed);  // the records have been read
   s.num = (int*)(ws + l.ctl + sizeof(otg::LvCtl));
-  for (int pass = 0; pass < 2 && e == cudaSuccess; ++pass) {
-    if (pass == 1 && n <= otg::kDigits + 1) break;  // a level has at least one pin
+  int pass = 0;
+  for (; !otg::sort_skip(n, pass) && e == cudaSuccess; ++pass) {  // n: a level has at least one pin
     e = otg::lv_launch(otg::levelize_hist, s.tiles, otg::ST, 0, pass > 0, st, a, s, pass);
     if (e == cudaSuccess)
       e = otg::lv_launch(otg::levelize_scan, 1, otg::kDigits, 0, true, st, a, s, pass);
     if (e == cudaSuccess)
       e = otg::lv_launch(otg::levelize_scatter, s.tiles, otg::ST, otg::kScatterSmem, true, st, a, s,
                          pass);
-    if (e == cudaSuccess && pass == 1)
-      e = otg::lv_launch(otg::levelize_ends, std::max(1, std::min((n + 255) / 256, 4 * d.sms)), 256,
-                         0, true, st, a, s);
   }
+  if (e == cudaSuccess && pass > 1)
+    e = otg::lv_launch(otg::levelize_ends, std::max(1, std::min((n + 255) / 256, 4 * d.sms)), 256,
+                       0, true, st, a, s);
   if (e == cudaSuccess) return OTG_OK;
   cudaGetLastError();
   return OTG_ERR_CUDA;
