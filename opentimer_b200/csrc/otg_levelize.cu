@@ -183,9 +183,10 @@ template <class Gp, class GetF>
 __device__ __forceinline__ void expand(const Gp& g, const LvArgs& a, const LvLists& ls, int m,
                                        int at, int threads, int L, GetF get) {
   const int lane = threadIdx.x & 31;
-  for (int i0 = at & ~31; i0 < 4 * m; i0 += threads) {
-    const int i = i0 + lane;
-    int x = i < 4 * m ? get(i >> 2, i & 3) : -1;
+  // unsigned: m and the threads' stride may add up to more than an int holds
+  for (unsigned k0 = (unsigned)(at & ~31) / 4; k0 < (unsigned)m; k0 += (unsigned)threads / 4) {
+    const unsigned k = k0 + (lane >> 2);
+    int x = k < (unsigned)m ? get((int)k, lane & 3) : -1;
     if (__any_sync(FULL, x == kWide)) {  // only a record's last word is kWide
       const bool wide = __shfl_sync(FULL, x, lane | 3) == kWide;
       const int e0 = __shfl_sync(FULL, x, lane & ~3), deg = __shfl_sync(FULL, x, (lane & ~3) | 1);
