@@ -287,13 +287,13 @@ otg_status otg_server_read(otg_server* s, int32_t design_id, int32_t* node2bfs, 
 /*
  * Tuning of the fused RC pass (per device; applies to later launches; no
  * counterpart in the reference, whose kernels have fixed launch shapes).
- * Nets of <= 32 nodes always take the warp path.  Block class c takes the
+ * Nets of <= 32 nodes always take the small-net kernel.  Block class c takes the
  * nets with class_max[c-1] < n <= class_max[c] (class_max[-1] = 32), one
  * CTA of class_threads[c] threads with class_items[c] scan items per
  * thread, in shared memory; nets above the last class_max take the
  * global-workspace path.  Shapes must be among the compiled ones
- * (threads x items: 64x4, 64x8, 128x4, 128x8, 256x2, 256x4, 256x8, 512x2,
- * 512x4, 512x8, 1024x2, 1024x4) and each class must fit shared memory.
+ * (threads x items: 32x4, 64x4, 64x8, 128x4, 128x8, 256x2, 256x4, 256x8,
+ * 512x2, 512x4, 512x8, 1024x2, 1024x4) and each class must fit shared memory.
  * Every valid tuning gives identical outputs; only the speed differs.
  * otg_rc_workspace_size depends on the tuning (the global-workspace
  * slices): size workspaces after setting it.

@@ -1130,18 +1130,19 @@ constexpr int kStaticSmemReserve = 2048;
 struct Shape {
   int T, K;
 };
-// The compiled block-class shapes (launch_shape dispatches on the index).
-constexpr Shape kShapeSet[] = {{64, 4},  {64, 8},  {128, 4}, {128, 8}, {256, 2},  {256, 4},
-                               {256, 8}, {512, 2}, {512, 4}, {512, 8}, {1024, 2}, {1024, 4}};
+// The compiled block-class shapes (launch_shape dispatches on the index); one
+// warp per net is the tile kernel's alone.
+constexpr Shape kShapeSet[] = {{64, 4},  {64, 8},  {128, 4}, {128, 8}, {256, 2},  {256, 4}, {256, 8},
+                               {512, 2}, {512, 4}, {512, 8}, {1024, 2}, {1024, 4}, {32, 4}};
 constexpr int kNumShapes = (int)(sizeof(kShapeSet) / sizeof(kShapeSet[0]));
 constexpr int kBlockClasses = 6;
 // Largest net of the tile kernel's classes; larger ones go to the huge class
 // (and, when there are few, to clusters).
 constexpr int kTileMax = 4888;
-// With many nets a class of nets up to this size runs one warp per net,
-// whatever its shape: nets of 33..64, 65..128, 129..200 nodes at 4.6, 6.2,
-// 7.4 nodes/ns against 3.0, 4.7, 6.9 with two warps; of 201..310 at 6.6
-// against 8.0.
+// With many nets the default table gives a class of nets up to this size one
+// warp per net: nets of 33..64, 65..128, 129..200 nodes at 4.6, 6.2, 7.4
+// nodes/ns against 3.0, 4.7, 6.9 with two warps; of 201..310 at 6.6 against
+// 8.0.
 constexpr int kWarpTileMax = 200;
 // Nets per SM of a pass up to which the default table gives a net more
 // threads (see default_tune).
@@ -1203,8 +1204,10 @@ RcTune default_tune(int smem_budget, long long nets, int max_net_nodes, int sms)
   // two of 512 on an SM (164,380 nets of 2..1500 nodes: 4.87 ms, 5.06 with
   // 1024 for 1232; 100,000 of 2..4096: 7.01 and 7.13, 7.38 with 256 threads
   // up to 2496)
-  constexpr Row many[] = {{128, {64, 4}},  {256, {64, 8}},   {512, {128, 8}},
-                          {1232, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
+  const Shape one = rc_use_tile() ? Shape{32, 4} : Shape{64, 4};
+  const Row many[] = {{128, one},       {256, max_net_nodes <= kWarpTileMax ? one : Shape{64, 8}},
+                      {512, {128, 8}},  {1232, {256, 4}},
+                      {2496, {512, 4}}, {0, {1024, 4}}};
   constexpr Row some[] = {{512, {128, 8}}, {1024, {256, 4}}, {2496, {512, 4}}, {0, {1024, 4}}};
   const Row few[] = {{512, {max_net_nodes <= 128 ? 128 : 256, 4}}, {1024, {512, 4}}, {0, {1024, 4}}};
   RcTune t;
@@ -1229,7 +1232,7 @@ bool tune_ok(const RcTune& t, int smem_budget) {
   for (int c = 0; c < t.num; ++c) {
     if (t.shape[c] < 0 || t.shape[c] >= kNumShapes || t.nmax[c] <= prev) return false;
     const Shape sh = kShapeSet[t.shape[c]];
-    if (rc_use_tile() && t.nmax[c] > kTileMax) return false;
+    if (rc_use_tile() ? t.nmax[c] > kTileMax : sh.T == 32) return false;
     if (rc_smem_bytes(t.nmax[c], sh.T, sh.K, rc_use_tile()) > (uint32_t)smem_budget) return false;
     prev = t.nmax[c];
   }
@@ -1439,11 +1442,8 @@ cudaError_t chain_launch(void (*kern)(P...), int grid, int block, size_t smem, i
 
 template <int T, int K>
 cudaError_t launch_smem_class(const RcJob& job, const int* list, int* count, int* work, int nmax,
-                              int sms, bool many, bool chained, cudaStream_t stream) {
+                              int sms, bool chained, cudaStream_t stream) {
   const bool tile = rc_use_tile();
-  if constexpr (T > 32)
-    if (tile && many && nmax <= kWarpTileMax)
-      return launch_smem_class<32, 4>(job, list, count, work, nmax, sms, many, chained, stream);
   auto kern = rc_block_kernel<T, K, uint16_t, true, true>;
   if constexpr (T > 32)
     if (!tile) kern = rc_block_kernel<T, K, uint16_t, true>;
@@ -1461,24 +1461,25 @@ cudaError_t launch_smem_class(const RcJob& job, const int* list, int* count, int
 }
 
 cudaError_t launch_shape(int s, const RcJob& job, const int* list, int* count, int* work,
-                         int nmax, int sms, bool many, bool chained, cudaStream_t st) {
+                         int nmax, int sms, bool chained, cudaStream_t st) {
   switch (s) {
-    case 0: return launch_smem_class<64, 4>(job, list, count, work, nmax, sms, many, chained, st);
-    case 1: return launch_smem_class<64, 8>(job, list, count, work, nmax, sms, many, chained, st);
-    case 2: return launch_smem_class<128, 4>(job, list, count, work, nmax, sms, many, chained, st);
-    case 3: return launch_smem_class<128, 8>(job, list, count, work, nmax, sms, many, chained, st);
-    case 4: return launch_smem_class<256, 2>(job, list, count, work, nmax, sms, many, chained, st);
-    case 5: return launch_smem_class<256, 4>(job, list, count, work, nmax, sms, many, chained, st);
-    case 6: return launch_smem_class<256, 8>(job, list, count, work, nmax, sms, many, chained, st);
-    case 7: return launch_smem_class<512, 2>(job, list, count, work, nmax, sms, many, chained, st);
-    case 8: return launch_smem_class<512, 4>(job, list, count, work, nmax, sms, many, chained, st);
-    case 9: return launch_smem_class<512, 8>(job, list, count, work, nmax, sms, many, chained, st);
-    case 10: return launch_smem_class<1024, 2>(job, list, count, work, nmax, sms, many, chained, st);
-    case 11: return launch_smem_class<1024, 4>(job, list, count, work, nmax, sms, many, chained, st);
+    case 0: return launch_smem_class<64, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 1: return launch_smem_class<64, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 2: return launch_smem_class<128, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 3: return launch_smem_class<128, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 4: return launch_smem_class<256, 2>(job, list, count, work, nmax, sms, chained, st);
+    case 5: return launch_smem_class<256, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 6: return launch_smem_class<256, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 7: return launch_smem_class<512, 2>(job, list, count, work, nmax, sms, chained, st);
+    case 8: return launch_smem_class<512, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 9: return launch_smem_class<512, 8>(job, list, count, work, nmax, sms, chained, st);
+    case 10: return launch_smem_class<1024, 2>(job, list, count, work, nmax, sms, chained, st);
+    case 11: return launch_smem_class<1024, 4>(job, list, count, work, nmax, sms, chained, st);
+    case 12: return launch_smem_class<32, 4>(job, list, count, work, nmax, sms, chained, st);
     default: return cudaErrorInvalidValue;
   }
 }
-static_assert(kNumShapes == 12, "launch_shape covers every kShapeSet entry");
+static_assert(kNumShapes == 13, "launch_shape covers every kShapeSet entry");
 
 RcArgs make_args(const otg_rc_forest* f, int* status) {
   RcArgs a;
@@ -1594,8 +1595,8 @@ otg_status rc_launch_job(RcJob job, int cap, int max_net_nodes, void* workspace,
     if (max_net_nodes <= cls.nmax[c - 1]) continue;
     const int nmax = std::min(cls.nmax[c], max_net_nodes);
     cudaStream_t st = next_stream();
-    err = launch_shape(tn.shape[c - 1], job, L(c), counters + c, work + c, nmax, di.sms,
-                       cap > kSomeNets * (long long)di.sms, chained, st);
+    err = launch_shape(tn.shape[c - 1], job, L(c), counters + c, work + c, nmax, di.sms, chained,
+                       st);
   }
   if (err == cudaSuccess) {
     cudaStream_t st = next_stream();
