@@ -68,6 +68,24 @@ def test_default_table_can_be_set(cuda, restore_tuning):
     assert otg.get_tuning() == t
 
 
+def test_one_warp_by_default(cuda, many, restore_tuning):
+    assert launched(cuda, many) == [32]
+    one = run(cuda, many)
+    otg.set_tuning(table([200], [64]))
+    assert launched(cuda, many) == [64]
+    two = run(cuda, many)
+    for k in OUT:
+        assert np.array_equal(one[k], two[k]), k
+    st, e, n2b, pid, _ = O.bfs(many)
+    assert st == 0
+    assert np.array_equal(one["node2bfs"], n2b) and np.array_equal(one["pid"], pid)
+    assert np.array_equal(one["edges"], e)
+    st, ref = O.elmore_f64(many)
+    assert st == 0
+    for q, r in zip(["load", "delay", "ldelay", "impulse"], ref):
+        assert elmore_err(many.nodes_start, bfs_local(many.nodes_start, n2b, one[q]), r) <= 1.0, q
+
+
 @pytest.mark.parametrize("sizes", [[33, 63, 64, 65, 129, 160, 161, 199, 200, 201, 1023, 1024, 1025],
                                    [2495, 3071, 4887, 4888]], ids=["small", "large"])
 @pytest.mark.parametrize("kind", ["rrt", "path", "star", "chain"])
