@@ -174,13 +174,20 @@ otg_status otg_levelize_status(const void* workspace, otg_stream_t stream);
  * with cached device buffers (grown, never shrunk) and pinned staging, and
  * stream large batches in chunks so transfers overlap compute.  Blocking.
  * Arrays as in otg_rc_forest but host pointers.
+ *
+ * The first otg_rc_timing_host call with 4 MB or more in pageable buffers of
+ * 256 KB or more allocates a 16 MB pinned ring and starts up to seven threads
+ * (fewer where std::thread::hardware_concurrency() is below eight), which
+ * copy between the ring and those buffers.  They sleep between calls and
+ * poll while a call copies.  Both stay until otg_release_host_context():
+ * call it before the library is unloaded.
  */
 otg_status otg_rc_timing_host(const otg_rc_forest* host_forest);
 otg_status otg_levelize_host(int32_t n, int32_t num_edges, const int32_t* fanin_start,
                              const int32_t* fanin, const int32_t* out_deg,
                              const int32_t* frontier0, int32_t first_size, int32_t* order,
                              int32_t* level, int32_t* level_ends, int32_t* counts);
-/* Frees the host-path context of the current device. */
+/* Frees the host-path context of the current device and ends its threads. */
 void otg_release_host_context(void);
 
 /*

@@ -215,8 +215,10 @@ bool pageable(const void* p) {
   return a.type == cudaMemoryTypeUnregistered;
 }
 
-// The copies, in order behind what stream s holds; those to the host are
-// complete on return, those to the device complete on s.
+// The copies, in order behind what stream s holds.  On return the caller's
+// pageable buffers have been read, or hold what came; the rest is on s, staged
+// copies to the device among it: up to kSlots of the ring's slots are still
+// being read then, and the next call waits for them.
 cudaError_t copy_all(Ctx* c, const std::vector<Copy>& copies, bool to_device, cudaStream_t s) {
   const cudaMemcpyKind kind = to_device ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
   std::vector<const Copy*> staged;
@@ -303,6 +305,10 @@ cudaError_t copy_all(Ctx* c, const std::vector<Copy>& copies, bool to_device, cu
       if (e != cudaSuccess) failed.store((int)e);
     }
   };
+  for (cudaEvent_t e : g.moved) {  // what the last call left in flight, maybe on another stream
+    const cudaError_t err = cudaEventSynchronize(e);
+    if (err != cudaSuccess) return err;
+  }
   const int hw = (int)std::max(2u, std::thread::hardware_concurrency());
   if (g.team->run(std::min(kLanes, hw), lane)) return (cudaError_t)failed.load();
   for (const Copy* k : staged) {  // no thread to be had
