@@ -55,9 +55,17 @@ namespace cg = cooperative_groups;
 constexpr unsigned FULL = 0xffffffffu;
 
 // A pin's fanins: up to four (-1: none), or {first index in fanin[], their
-// number, 0, kWide}.  In the lists a wide record names at most kWideMax
-// fanins, a quad of lanes' worth, unless it has more than kWideLong.
-constexpr int kWide = -2, kWideMax = 4, kWideLong = 64;
+// number, 0, kWide}.  In the lists a wide pin takes several records: of a quad
+// of lanes' worth of fanins, up to kWideLong; beyond (a driver's sinks, where
+// the fanouts are levelized) of a warp's worth, or twice that and so on, at
+// most kWideRecs.  In one record a warp went through such a pin by itself: a
+// pin of 12,000 fanins in a graph of 24,000 pins took 397 us, now 118 (510
+// and 91 on the grid), one of 100,000 3.4 ms and 0.77.
+constexpr int kWide = -2, kWideMax = 4, kWideLong = 64, kWideRecs = 512, kWideStay = 32;
+// log2 of a record's fanins
+__device__ __forceinline__ int wide_shift(int deg) {
+  return deg <= kWideLong ? 2 : max(5, 32 - __clz((deg - 1) / kWideRecs));
+}
 
 struct LvCtl {
   GridCtl grid;
@@ -116,11 +124,11 @@ struct LvLists {
 __device__ __forceinline__ bool put_records(int4* rec, int* pin, int cap, int at, int recs, int v,
                                             int4 pk) {
   const bool fits = at + recs <= cap;
+  const int len = recs > 1 ? 1 << wide_shift(pk.y) : 0;
   for (int k = 0; k < recs; ++k) {
     if (at + k >= cap) break;
     int4 x = pk;
-    if (recs > 1)
-      x = make_int4(pk.x + kWideMax * k, min(kWideMax, pk.y - kWideMax * k), 0, kWide);
+    if (recs > 1) x = make_int4(pk.x + len * k, min(len, pk.y - len * k), 0, kWide);
     rec[at + k] = fits ? x : make_int4(-1, -1, -1, -1);
     pin[at + k] = fits && k == 0 ? v : -1;
   }
@@ -151,11 +159,15 @@ __device__ __forceinline__ void decrement(const Gp& g, const LvArgs& a, const Lv
   }
   const unsigned set = __ballot_sync(FULL, ready);
   if (set == 0u) return;
-  const int recs =
-      !ready ? 0
-             : (pk.w == kWide && pk.y <= kWideLong ? (pk.y + kWideMax - 1) / kWideMax : 1);
+  int recs = ready ? 1 : 0;
+  if (ready && pk.w == kWide) {
+    const int s = wide_shift(pk.y);
+    recs = (int)((unsigned)(pk.y - 1) >> s) + 1;
+  }
   int at = __popc(set & ((1u << lane) - 1u)), total = __popc(set);
+  bool stay = false;
   if (__any_sync(FULL, recs > 1)) {
+    if constexpr (Gp::kKeepLong) stay = __any_sync(FULL, recs > kWideStay);
     int upto = recs;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -167,7 +179,7 @@ __device__ __forceinline__ void decrement(const Gp& g, const LvArgs& a, const Lv
   }
   int* len = g.length(L);
   int base = -1;
-  if (lane == 0 && *(volatile int*)len < g.most()) base = atomicAdd(len, total);
+  if (lane == 0 && (*(volatile int*)len < g.most() || stay)) base = atomicAdd(len, total);
   base = __shfl_sync(FULL, base, 0);
   if (ready) {
     if (base < 0) g.hand_on(v, pk, recs, L);
@@ -263,6 +275,7 @@ struct ClGroup {
   }
   __device__ int* length(int L) const { return &sw.len[L & 3]; }
   __device__ int most() const { return kLocalMax; }
+  static constexpr bool kKeepLong = false;  // another CTA's list is as good
   __device__ void spill(int v, int L) const {
     spill_pin(a, v, L);
     for (int i = 0; i < (1 << sshift); ++i) *cl.map_shared_rank(&sw.ovf[L & 3], i) = 1;
@@ -379,11 +392,15 @@ struct GridWait {
 
 struct GridGroup {
   const LvArgs& a;
+  const LvLists& ls;
   int* len;         // by level parity
   const int* room;  // entries before a warp puts pins on the spill list
   __device__ int* counter(int v) const { return a.cnt + v; }
   __device__ int* length(int L) const { return len + (L & 1); }
   __device__ int most() const { return *room; }
+  // the list spreads a very long pin (kWideStay records) over the CTA's warps,
+  // the spill list does not
+  static constexpr bool kKeepLong = true;
   __device__ void spill(int v, int L) const { spill_pin(a, v, L); }
   __device__ void hand_on(int v, int4, int, int L) const { spill_pin(a, v, L); }
 };
@@ -394,7 +411,7 @@ __global__ void __launch_bounds__(LT, 1) levelize_grid_kernel(LvArgs a) {
   const int G = gridDim.x, tid = threadIdx.x;
   const int gtid = blockIdx.x * LT + tid, gstride = G * LT;
   const LvLists ls{(int4*)lv_sm, (int*)((int4*)lv_sm + 2 * kGridCap), kGridCap};
-  const GridGroup g{a, s_len, &s_room};
+  const GridGroup g{a, ls, s_len, &s_room};
   GridWait barrier{&a.ctl->grid};
   if (tid < 2) s_len[tid] = 0;
   if (tid == 0) {
