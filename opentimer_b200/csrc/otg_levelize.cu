@@ -467,7 +467,8 @@ __global__ void __launch_bounds__(LT, 1) levelize_grid_kernel(LvArgs a) {
 // consecutive items, a scan and a scatter.  A pass whose digit is 0 for every
 // level is left out: its kernels return at once, and where the graph has too
 // few pins for so many levels, they are not launched.
-constexpr int kDigitBits = 10, kDigits = 1 << kDigitBits, kMaxTiles = 256, ST = 1024;
+constexpr int kDigitBits = 10, kDigits = 1 << kDigitBits, kMinTiles = 6, kMaxTiles = 256,
+              ST = 1024;
 
 struct LvSort {
   int per;      // items per tile
@@ -578,7 +579,8 @@ __global__ void __launch_bounds__(ST) levelize_scatter(LvArgs a, LvSort s, int p
   for (int d = threadIdx.x; d < kDigits; d += ST) base[d] = s.hist[d * s.tiles + blockIdx.x];
   __syncthreads();
   // each warp takes consecutive items, 32 at a time
-  const int per = s.per / (ST / 32), b = blockIdx.x * s.per + w * per;
+  const int b = blockIdx.x * s.per + w * (s.per / (ST / 32));
+  const int per = min(s.per / (ST / 32), (pass == 0 ? a.n : *s.num) - b);
   uint16_t* mine = cnt + w * kDigits;
   for (int i = 0; i < per; i += 32) {
     int v;
@@ -742,11 +744,15 @@ ClPlan lv_cluster_plan(int n, const LvDev& d) {
 
 size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// Items per sort tile: a multiple of 32 per warp, about kMaxTiles tiles at
-// most, and no more than the scatter's 16-bit counts hold.
+// Items per sort tile: a multiple of 32 per warp, and no more than the
+// scatter's 16-bit counts hold.  About kMinTiles tiles while these are small
+// (one CTA for all takes as long as 8,192 pins whatever their number: 200 pins
+// / 3 levels 31 us, now 21; 8,000 45 and 39), then kMaxTiles at most (the scan
+// reads them one after another: 60k gates 813 us with tiles of 1,024, 686).
 LvSort lv_tiles(int n) {
   LvSort s{};
-  s.per = 8 * ST;
+  s.per = ST;
+  while (s.per < 8 * ST && (long long)s.per * kMinTiles < n) s.per += ST;
   while (s.per < 63 * ST && (long long)s.per * kMaxTiles < n) s.per += ST;
   s.tiles = std::max(1, (int)(((long long)n + s.per - 1) / s.per));
   return s;
