@@ -173,7 +173,7 @@ __device__ __forceinline__ void rc_nets_small(const RcArgs& a, int net, int b, i
   rows(a.load);
   if (n > 0) {
     f64(sum, 0) = 0.0;
-    f32(acc, 0) = 0.0f;  // cap * delay at the root
+    f32(acc, 0) = __fmul_rn(f32(acc, 0), 0.0f);  // cap * delay at the root; not 0 for every cap
   }
   {
     const uint2* mp = sm.meta + c + C;
