@@ -35,12 +35,11 @@ TUNE_NETS = 50_000
 SPEF_NETS = 20_000
 # DRAM bytes per node of one RC pass (dram__bytes_read.sum + dram__bytes_write.sum
 # over the 8 launches of one pass), from an ncu capture of 30k nets of the same
-# net-size distribution with the autotuned table: 2.204 GB / 15,951,150 nodes
+# net-size distribution with the autotuned table: 2.324 GB / 15,951,150 nodes
 # (profiles/rc_pass_dram_traffic_30k_nets.md).  The pass's traffic grows with
 # its nodes, so a step's traffic is this times the step's nodes.  (At 30k nets
-# part of the small classes' writes is still in L2 when the capture ends; the
-# dominant kernel alone moves 152.8 B/node.)
-RC_DRAM_BYTES_PER_NODE = 138.2
+# part of the small classes' writes is still in L2 when the capture ends.)
+RC_DRAM_BYTES_PER_NODE = 145.7
 FU_GATES = 50_000
 FU_REPS = 5
 FU_CHANGE = 0.01  # fraction of the nets a change SPEF re-draws
@@ -48,8 +47,8 @@ FU_CHANGE = 0.01  # fraction of the nets a change SPEF re-draws
 INC_GATES, INC_ITERS, INC_FRAC, INC_PLAIN_ITERS, INC_REF_ITERS = 200_000, 1000, 0.005, 100, 3
 # serving
 SRV_DESIGNS, SRV_PINS_LO, SRV_PINS_HI = 16, 10_000, 2_000_000
-# offered rates: below both paths' capacity, between the plain path's (about
-# 180 req/s on the 16 designs) and the batched one's (about 450), and above both
+# offered rates: two below both paths' capacity (on the 16 designs about 480
+# req/s one at a time, 870 batched), and one above both
 SRV_RATES, SRV_MAX_REQ, SRV_SAT_REQ, SRV_REF_REQ = (100, 300, 1_000), 2_000, 3_000, 12
 SRV_PINS_PER_GATE = 2.75  # designgen: pins per gate of a design
 
@@ -442,7 +441,7 @@ def run_ours(args, world, rank, local):
     return line
 
 
-PARITY_BINS = (2, 33, 129, 257, 513, 1025, 2049, 4097)  # warp path, then block classes
+PARITY_BINS = (2, 33, 129, 257, 513, 1025, 2049, 4097)  # small nets, then block classes
 PARITY_NETS_PER_BIN = 300
 
 
@@ -1253,8 +1252,9 @@ def run_huge():
         res["outputs_identical"] = all(torch.equal(x, y) for x, y in
                                        zip(outs["one_cta_per_net"], outs["default"]))
         out[name] = res
-    out["what"] = ("default: clusters of 8 CTAs per net when the device-side count of huge nets "
-                   "is at most 2 per cluster, else one CTA per net")
+    out["what"] = ("default: clusters of 8 CTAs per net (16 in a pass of at most four nets) when "
+                   "the device-side count of huge nets is one that clusters finish sooner, else "
+                   "one CTA per net")
     return out
 
 

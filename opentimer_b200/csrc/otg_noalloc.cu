@@ -28,7 +28,7 @@
 //   * It never calls cudaMalloc, cudaFree or any other allocating routine.
 //   * Limit: the workspace of the batch must fit 16 MiB, i.e. at most
 //     524,284 nets per call, and every net within the shared-memory classes
-//     of the device's tuning (4,265 nodes on a B200 with the default
+//     of the device's tuning (4,888 nodes on a B200 with the default
 //     tuning; otg_rc_set_tuning moves the bound); anything larger returns
 //     OTG_ERR_WORKSPACE before launching.
 #include <cuda_runtime.h>

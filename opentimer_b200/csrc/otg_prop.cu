@@ -163,7 +163,8 @@ __device__ __noinline__ float timing_value(const LutSrc& src, const Lut& m, floa
 // three fused multiply-adds.  In exact arithmetic the same bilinear form as
 // lut_eval's, whichever axis comes first; both lines start at the nearer end
 // of their segment.  Slew axes of up to kPrepAxis entries; others go through
-// timing_value.  After the wait an arc's two tables take about 250 cycles of
+// timing_value, and so do queries that have no finite answer this way (see
+// fprop_warp).  After the wait an arc's two tables take about 250 cycles of
 // every gate on a path; interpolating both axes there with lut_eval took 1700
 // (six divisions, each with its own branch), and two calls of timing_value
 // 3500.  Reducing the tables to the load before the wait leaves one entry

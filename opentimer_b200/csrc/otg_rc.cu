@@ -1131,13 +1131,16 @@ struct Shape {
   int T, K;
 };
 // The compiled block-class shapes (launch_shape dispatches on the index); one
-// warp per net is the tile kernel's alone.
+// warp per net is the tile kernel's alone.  K counts on the legacy block path
+// only: the tile kernel's items per thread follow from the net.
 constexpr Shape kShapeSet[] = {{64, 4},  {64, 8},  {128, 4}, {128, 8}, {256, 2},  {256, 4}, {256, 8},
                                {512, 2}, {512, 4}, {512, 8}, {1024, 2}, {1024, 4}, {32, 4}};
 constexpr int kNumShapes = (int)(sizeof(kShapeSet) / sizeof(kShapeSet[0]));
 constexpr int kBlockClasses = 6;
-// Largest net of the tile kernel's classes; larger ones go to the huge class
-// (and, when there are few, to clusters).
+// Largest net of the tile kernel's classes, and the largest bound a tuning may
+// name; larger nets go to the huge class (and, when there are few, to
+// clusters).  The layout would hold 5,105 nodes in shared memory: this is what
+// it held when tunings were first accepted, and the bound callers know.
 constexpr int kTileMax = 4888;
 // With many nets the default table gives a class of nets up to this size one
 // warp per net: nets of 33..64, 65..128, 129..200 nodes at 4.6, 6.2, 7.4
@@ -1518,7 +1521,8 @@ bool forest_ok(const otg_rc_forest* f) {
 // CTAs of the small-net kernel, one warp each: as many as its nets take in
 // one go, eight of up to 16 nodes, four of larger ones (with eight, 2,243 nets
 // of 2..24 nodes took two: 30.5 us against 18.5), and one net each where there
-// are few (300 nets of 2..24 nodes 16.8 us, of 2..32 20.6 against 22.6).
+// are few (300 nets of 2..24 nodes 16.8 us, of 2..32 20.6 against 22.6).  Nets
+// of up to 16 nodes always share a warp: fewer to one have not been measured.
 int small_ctas(int nets, int max_net_nodes, int sms) {
   const int k = max_net_nodes <= kSmallCells / 8 ? 8 : (nets > 4 * sms ? 4 : 1);
   return std::max(1, std::min((nets + k - 1) / k, kSmallCtas * sms));

@@ -19,9 +19,9 @@
 // the warp takes one net, and its sweeps are O(n) shuffles each (337 us for
 // 250,000 nets of 2..16 nodes with sinks; now 152 us).  One lane per net
 // runs fewer instructions but leaves six warps per SM, too few to hide the
-// serial sweeps (261 us).  What bounds it: the load/store unit (about 13
-// shared-memory and L1 wavefronts per node, 75% busy; 16-byte cells packed
-// without columns cost 16) and the sweeps' latency; HBM is at a quarter.
+// serial sweeps (261 us).  What bounds it: the load/store unit (15 wavefronts
+// per node, 12 of them in shared memory, 85% busy) and the sweeps' latency;
+// HBM is at a fifth.
 constexpr int kSmallMax = 32;     // largest net: one mask bit per node
 constexpr int kSmallCells = 128;  // cells of a warp's slice
 constexpr int kSmallCtas = 22;  // one-warp CTAs per SM that the slices allow
