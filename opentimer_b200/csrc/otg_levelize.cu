@@ -31,7 +31,7 @@
 //            so the kernel always returns and the host sees OTG_ERR_TIMEOUT.
 // Before, a level's pins were found in ready bitmaps, written out in order,
 // and their fanins looked up, scanned and searched by thread, all on the
-// chain: 2.53 ms on 5M pins / 200 levels (grid; now 1.47), 1.30 ms on a
+// chain: 2.53 ms on 5M pins / 200 levels (grid; now 1.5), 1.30 ms on a
 // 60k-gate design's 163k pins / 374 levels (cluster; now 0.55).  What bounds
 // it now is the chain still: per level one barrier, one counter round trip
 // and the appends, 1.4 us in the cluster and 2.6 us on the grid where a
@@ -392,14 +392,13 @@ struct GridWait {
 
 struct GridGroup {
   const LvArgs& a;
-  const LvLists& ls;
   int* len;         // by level parity
   const int* room;  // entries before a warp puts pins on the spill list
   __device__ int* counter(int v) const { return a.cnt + v; }
   __device__ int* length(int L) const { return len + (L & 1); }
   __device__ int most() const { return *room; }
-  // the list spreads a very long pin (kWideStay records) over the CTA's warps,
-  // the spill list does not
+  // the list spreads a very long pin (over kWideStay records) over the CTA's
+  // warps, the spill list does not
   static constexpr bool kKeepLong = true;
   __device__ void spill(int v, int L) const { spill_pin(a, v, L); }
   __device__ void hand_on(int v, int4, int, int L) const { spill_pin(a, v, L); }
@@ -411,7 +410,7 @@ __global__ void __launch_bounds__(LT, 1) levelize_grid_kernel(LvArgs a) {
   const int G = gridDim.x, tid = threadIdx.x;
   const int gtid = blockIdx.x * LT + tid, gstride = G * LT;
   const LvLists ls{(int4*)lv_sm, (int*)((int4*)lv_sm + 2 * kGridCap), kGridCap};
-  const GridGroup g{a, ls, s_len, &s_room};
+  const GridGroup g{a, s_len, &s_room};
   GridWait barrier{&a.ctl->grid};
   if (tid < 2) s_len[tid] = 0;
   if (tid == 0) {
